@@ -527,7 +527,8 @@ struct mhd_problem {
     a.op = op;
     a.step = dstep;
     a.stage = stage;
-    a.hydro = p.hydro_only;
+    a.vpen = p.vp != 0;
+    a.forced = forced();
     const double n3 = (double)g.n * g.n * g.n;
     a.pscale = (float)(1.0 / (n3 * n3));
     a.vscale = (float)(1.0 / n3);
@@ -540,28 +541,23 @@ struct mhd_problem {
   // Hermitian part of X's kx = 0 plane was copied out into aux by the z_forward before it)
   int epilogue(const float2* X, float2* xn, int op, float hf, float ca, float cb, BatchRef br, int stage) {
     const RkArgs a = rk_args(X, xn, op, hf, ca, cb, stage);
-    const int bx = g.kx <= 256 ? (g.kx + 31) / 32 * 32 : 256;
-    const dim3 grid((g.kx + bx - 1) / bx, g.k2, g.k2 * cap);
-    const bool f = forced(), v = p.vp != 0;
+    const dim3 grid((unsigned)((FS() / 2 + kStageThreads - 1) / kStageThreads), hd_form() ? 1 : 2, cap);
     return launch(KC_RKEPI, [&] {
-      if (hd_form() && v) launch_epilogue<false, true, true>(op, grid, bx, a, br);
-      else if (hd_form()) launch_epilogue<false, false, true>(op, grid, bx, a, br);
-      else if (f && v) launch_epilogue<true, true>(op, grid, bx, a, br);
-      else if (f) launch_epilogue<true, false>(op, grid, bx, a, br);
-      else if (v) launch_epilogue<false, true>(op, grid, bx, a, br);
-      else launch_epilogue<false, false>(op, grid, bx, a, br);
+      if (hd_form()) launch_epilogue<true, true>(op, grid, a, br);
+      else if (a.vpen || a.forced) launch_epilogue<true, false>(op, grid, a, br);
+      else launch_epilogue<false, false>(op, grid, a, br);
     });
   }
-  // record: the stage whose physical fields getCFL! reads (the last one of a step)
-  template <bool F, bool V, bool H = false>
-  void launch_epilogue(int op, dim3 grid, int bx, const RkArgs& a, BatchRef br) {
+  template <bool G, bool H>
+  void launch_epilogue(int op, dim3 grid, const RkArgs& a, BatchRef br) {
+    constexpr int T = kStageThreads;
     switch (op) {
-      case OP_RHS: rk_epilogue_kernel<OP_RHS, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
-      case OP_RK4_FIRST: rk_epilogue_kernel<OP_RK4_FIRST, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
-      case OP_RK4_MID: rk_epilogue_kernel<OP_RK4_MID, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
-      case OP_RK4_LAST: rk_epilogue_kernel<OP_RK4_LAST, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
-      case OP_LS_FIRST: rk_epilogue_kernel<OP_LS_FIRST, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
-      default: rk_epilogue_kernel<OP_LS, F, V, H><<<grid, bx, 0, stream>>>(a, g, br); break;
+      case OP_RHS: stage_kernel<OP_RHS, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
+      case OP_RK4_FIRST: stage_kernel<OP_RK4_FIRST, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
+      case OP_RK4_MID: stage_kernel<OP_RK4_MID, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
+      case OP_RK4_LAST: stage_kernel<OP_RK4_LAST, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
+      case OP_LS_FIRST: stage_kernel<OP_LS_FIRST, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
+      default: stage_kernel<OP_LS, G, H><<<grid, T, 0, stream>>>(a, g, br); break;
     }
   }
   // DivVCorrection! / DivBCorrection! of the slots in br (mask: 1 u, 2 B)

@@ -8,9 +8,9 @@ namespace mhdgb {
 // Runge-Kutta stage operations of the epilogue.
 enum StageOp : int {
   OP_RHS = 0,       // out <- R
-  OP_RK4_FIRST = 1, // acc <- R/6 ; xn <- sol + h R            (X = sol)
-  OP_RK4_MID = 2,   // acc <- acc + R/3 ; xn <- sol + h R
-  OP_RK4_LAST = 3,  // sol <- sol + dt (acc + R/6)
+  OP_RK4_FIRST = 1, // acc <- R ; xn <- sol + h R              (X = sol)
+  OP_RK4_MID = 2,   // acc <- acc + 2 R ; xn <- sol + h R
+  OP_RK4_LAST = 3,  // sol <- sol + dt/6 (acc + R)
   OP_LS_FIRST = 4,  // du <- dt R ; u <- u + b du              (X = u)
   OP_LS = 5,        // du <- a du + dt R ; u <- u + b du
 };
@@ -38,8 +38,8 @@ struct RkArgs {
   int op;
   const long long* step; // per-slot step counters (random forcing: call = 8 * step + stage)
   int stage;             // right-hand-side evaluation within the step (7: outside a step)
-  int hydro;             // hydrodynamics: the induction right-hand side is zero, B stays zero
   float vscale;          // 1/n^3: the penalty planes are n^3 times the reference's rfft
+  int vpen, forced;      // penalty planes present, forcing on for some slot
 };
 
 // ------------------------------------------------------------------------------------------
@@ -89,128 +89,100 @@ struct RkSlot {
   float2* sol;
   float2* acc;
   float2* xn;
-  float h, dt, ca, cb;
+  float h, dt, dt6, ca, cb;  // dt6 = dt / 6
 };
 
-template <int OP>
-__device__ __forceinline__ void rk_apply(const RkSlot& a, long long o, float2 x, float2 R) {
-  if constexpr (OP == OP_RHS) {
-    a.acc[o] = R;
-  } else if constexpr (OP == OP_RK4_FIRST) {
-    a.acc[o] = make_float2(R.x / 6.f, R.y / 6.f);
-    a.xn[o] = make_float2(x.x + a.h * R.x, x.y + a.h * R.y);
-  } else if constexpr (OP == OP_RK4_MID) {
-    const float2 s = a.sol[o], q = a.acc[o];
-    a.acc[o] = make_float2(q.x + R.x / 3.f, q.y + R.y / 3.f);
-    a.xn[o] = make_float2(s.x + a.h * R.x, s.y + a.h * R.y);
-  } else if constexpr (OP == OP_RK4_LAST) {
-    const float2 s = a.sol[o], q = a.acc[o];
-    const float2 tot = make_float2(q.x + R.x / 6.f, q.y + R.y / 6.f);
-    a.sol[o] = make_float2(s.x + a.dt * tot.x, s.y + a.dt * tot.y);
-  } else if constexpr (OP == OP_LS_FIRST) {
-    const float2 du = make_float2(a.dt * R.x, a.dt * R.y);
-    a.acc[o] = du;
-    a.xn[o] = make_float2(x.x + a.cb * du.x, x.y + a.cb * du.y);
-  } else if constexpr (OP == OP_LS) {
-    const float2 q = a.acc[o];
-    const float2 du = make_float2(a.ca * q.x + a.dt * R.x, a.ca * q.y + a.dt * R.y);
-    a.acc[o] = du;
-    a.xn[o] = make_float2(x.x + a.cb * du.x, x.y + a.cb * du.y);
-  }
-}
-
-
-// The stress and induction sums of one retained mode (already scaled to the reference's rfft):
+// The right-hand side of one retained mode, a triple (u or B) at a time:
 // V = (kx Dxz + ky Txy + kz Txz, kx Txy + ky Dyz + kz Tyz, kx Txz + ky Tyz) and
 // W = k x E with E = (Ayz, -Axz, Axy): Wx = ky Axy + kz Axz, Wy = kz Ayz - kx Axy,
 // Wz = -(kx Axz + ky Ayz).  The nonlinear terms are i (V - k (k.V)/k^2) and i W.
-struct ModeSums {
-  float2 Vx, Vy, Vz, Wx, Wy, Wz;
-};
-
-// The right-hand side of one retained mode (jz, jy, x) of a slot from its sums, the stage state
-// (the kx = 0 plane diffuses its Hermitian part), volume penalisation, forcing, and the stage
-// update.  i is the mode's offset in a compact field; prod the slot's product planes (VPEN only).
-template <int OP, bool FORCED, bool VPEN, bool HD>
-__device__ __forceinline__ void finish_mode(const RkArgs& a, const Geom& geo, int slot, int jz, int jy, int x, long long i,
-                                            float kxv, float kyv, float kzv, const ModeSums& m, const float2* prod) {
-  constexpr int NF = HD ? 3 : 6;
-  const long long fs = a.fs;
-  const SlotParams sp = a.sp[slot];
-  const long long so = slot * a.stI;
-  RkSlot rs{a.sol + so, a.acc + so, a.xn + so, a.hf * sp.dt, sp.dt, a.ca, a.cb};
-  const float2* X = a.X + so;
+// Volume penalisation (VP_UᵢUpdate! / VP_BᵢUpdate!, src/Solver/VPSolver.jl:20-58):
+// N_a += -(δ_aj - k_a k_j / k^2) F_j with F = rfft(chi / eta (u - U0)) (and chi / eta (B - B0)),
+// eta = 13 dt / 7, 1/k^2 = 0 at k = 0.  MHD: the six penalty planes are 8..13 (u x, u y, u z, B x,
+// B y, B z), n^3 times the reference's rfft; the hydrodynamic form keeps u in the spare product
+// slots 6, 7, 5 (x, y, z) at the products' scale, n^6.
+// Forcing (addforcing!): N[u] += F, then the kx = 0 plane keeps its real part.
+//
+// Right-hand side of field triple t (0: u, 1: B) at one retained mode from its product
+// planes (p[0..5) = Dxz Dyz Txy Txz Tyz, or p[0..3) = Axy Axz Ayz), with the formulas above.  GENERAL: penalty planes (a.vpen) and forcing (a.forced).
+template <bool GENERAL, bool HD>
+__device__ __forceinline__ void triple_rhs(const RkArgs& a, const Geom& geo, const SlotParams& sp, int slot, int t, int x, int jy,
+                                           int jz, float kxv, float kyv, float kzv, const float2 (&xd)[3], const float2 (&p)[5],
+                                           const float2 (&pen)[3], float2 (&R)[3]) {
+  // the products' scale goes with the wavenumbers of the sums (three factors per mode)
+  const float sx = a.pscale * kxv, sy = a.pscale * kyv, sz = a.pscale * kzv;
   const float k2 = kxv * kxv + kyv * kyv + kzv * kzv;
-  float2 xv[6], xd[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) xv[c] = xd[c] = c < NF ? X[c * fs + i] : make_float2(0.f, 0.f);
-  if (x == 0) {
-    const long long p = (long long)jz * geo.k2 + jy, pl = (long long)geo.k2 * geo.k2;
-    const float2* H = a.H + slot * a.hI;
-#pragma unroll
-    for (int c = 0; c < NF; ++c) xd[c] = H[c * pl + p];
-  }
   const float ik2 = k2 > 0.f ? 1.0f / k2 : 0.f;
-  const float kvx = (kxv * m.Vx.x + kyv * m.Vy.x + kzv * m.Vz.x) * ik2;
-  const float kvy = (kxv * m.Vx.y + kyv * m.Vy.y + kzv * m.Vz.y) * ik2;
-  float2 nl[6];
-  nl[0] = make_float2(-(m.Vx.y - kxv * kvy), m.Vx.x - kxv * kvx);
-  nl[1] = make_float2(-(m.Vy.y - kyv * kvy), m.Vy.x - kyv * kvx);
-  nl[2] = make_float2(-(m.Vz.y - kzv * kvy), m.Vz.x - kzv * kvx);
-  nl[3] = make_float2(-m.Wx.y, m.Wx.x);
-  nl[4] = make_float2(-m.Wy.y, m.Wy.x);
-  nl[5] = make_float2(-m.Wz.y, m.Wz.x);
-  const float du = -sp.nu * k2, db = -sp.eta * k2;
-  float2 R[6];
+  const float ks[3] = {kxv, kyv, kzv};
+  float2 nl[3];
+  if (t == 0) {
+    const float2 dxz = p[0], dyz = p[1], txy = p[2], txz = p[3], tyz = p[4];
+    const float2 V[3] = {make_float2(sx * dxz.x + sy * txy.x + sz * txz.x, sx * dxz.y + sy * txy.y + sz * txz.y),
+                         make_float2(sx * txy.x + sy * dyz.x + sz * tyz.x, sx * txy.y + sy * dyz.y + sz * tyz.y),
+                         make_float2(sx * txz.x + sy * tyz.x, sx * txz.y + sy * tyz.y)};
+    const float kvx = (kxv * V[0].x + kyv * V[1].x + kzv * V[2].x) * ik2;
+    const float kvy = (kxv * V[0].y + kyv * V[1].y + kzv * V[2].y) * ik2;
 #pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    const float dk = c < 3 ? du : db;
-    R[c] = make_float2(nl[c].x + dk * xd[c].x, nl[c].y + dk * xd[c].y);
+    for (int c = 0; c < 3; ++c) nl[c] = make_float2(-(V[c].y - ks[c] * kvy), V[c].x - ks[c] * kvx);
+  } else {
+    const float2 axy = p[0], axz = p[1], ayz = p[2];
+    const float2 Wc[3] = {make_float2(sy * axy.x + sz * axz.x, sy * axy.y + sz * axz.y),
+                          make_float2(sz * ayz.x - sx * axy.x, sz * ayz.y - sx * axy.y),
+                          make_float2(-(sx * axz.x + sy * ayz.x), -(sx * axz.y + sy * ayz.y))};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nl[c] = make_float2(-Wc[c].y, Wc[c].x);
   }
-  if constexpr (VPEN) {
-    // VP_UᵢUpdate! / VP_BᵢUpdate! (src/Solver/VPSolver.jl:20-58): N_a += -(δ_aj - k_a k_j / k^2) F_j
-    // with F = rfft(chi / eta (u - U0)) (and chi / eta (B - B0)), eta = 13 dt / 7, 1/k^2 = 0 at k = 0
-    // MHD: the six penalty planes are 8..13 (u x, u y, u z, B x, B y, B z), n^3 times the
-    // reference's rfft; the hydrodynamic form keeps u in the spare product slots 6, 7, 5 (x, y, z)
-    // at the products' scale, n^6
-    const float sc = -(HD ? a.pscale : a.vscale) * 7.f / (13.f * sp.dt);
-    float2 F[6];
+  const float dk = -(t == 0 ? sp.nu : sp.eta) * k2;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      const int plane = HD ? (q == 0 ? 6 : q == 1 ? 7 : 5) : 8 + q;
-      F[q] = (HD && q >= 3) ? make_float2(0.f, 0.f) : cscale(__ldcs(prod + plane * fs + i), sc);
+  for (int c = 0; c < 3; ++c) R[c] = make_float2(nl[c].x + dk * xd[c].x, nl[c].y + dk * xd[c].y);
+  if constexpr (GENERAL) {
+    if (a.vpen) {  // N_a += -(delta_aj - k_a k_j / k^2) F_j of this triple
+      const float sc = -(HD ? a.pscale : a.vscale) * 7.f / (13.f * sp.dt);
+      const float2 f[3] = {cscale(pen[0], sc), cscale(pen[1], sc), cscale(pen[2], sc)};
+      const float px = (kxv * f[0].x + kyv * f[1].x + kzv * f[2].x) * ik2;
+      const float py = (kxv * f[0].y + kyv * f[1].y + kzv * f[2].y) * ik2;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) R[c] = make_float2(R[c].x + f[c].x - ks[c] * px, R[c].y + f[c].y - ks[c] * py);
     }
+    if (!HD && a.forced && t == 0 && sp.fA != 0.f) {
+      const unsigned long long call = 8ull * (unsigned long long)a.step[slot] + (unsigned long long)a.stage;
+      const unsigned long long key = mix64(sp.fseed ^ mix64(call));
+      const int nkr = geo.n / 2 + 1;
+      const unsigned long long index =
+          (unsigned long long)x + (unsigned long long)nkr * ((unsigned long long)freq_of_kept(geo, jy) +
+                                                              (unsigned long long)geo.n * freq_of_kept(geo, jz));
+      float2 F[3];
+      a99_force(sp, key, index, kxv, kyv, kzv, F);
 #pragma unroll
-    for (int h = 0; h < (HD ? 1 : 2); ++h) {
-      const float2 f0 = F[3 * h], f1 = F[3 * h + 1], f2 = F[3 * h + 2];
-      const float px = (kxv * f0.x + kyv * f1.x + kzv * f2.x) * ik2;
-      const float py = (kxv * f0.y + kyv * f1.y + kzv * f2.y) * ik2;
-      R[3 * h] = make_float2(R[3 * h].x + f0.x - kxv * px, R[3 * h].y + f0.y - kxv * py);
-      R[3 * h + 1] = make_float2(R[3 * h + 1].x + f1.x - kyv * px, R[3 * h + 1].y + f1.y - kyv * py);
-      R[3 * h + 2] = make_float2(R[3 * h + 2].x + f2.x - kzv * px, R[3 * h + 2].y + f2.y - kzv * py);
-    }
-  }
-  if (FORCED && sp.fA != 0.f) {  // addforcing!: N[u] += F, then the kx = 0 plane keeps its real part
-    const unsigned long long call = 8ull * (unsigned long long)a.step[slot] + (unsigned long long)a.stage;
-    const unsigned long long key = mix64(sp.fseed ^ mix64(call));
-    const int nkr = geo.n / 2 + 1;
-    const unsigned long long index =
-        (unsigned long long)x + (unsigned long long)nkr * ((unsigned long long)freq_of_kept(geo, jy) +
-                                                            (unsigned long long)geo.n * freq_of_kept(geo, jz));
-    float2 F[3];
-    a99_force(sp, key, index, kxv, kyv, kzv, F);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      R[c] = make_float2(R[c].x + F[c].x, R[c].y + F[c].y);
-      if (x == 0) R[c].y = 0.f;
+      for (int c = 0; c < 3; ++c) {
+        R[c] = make_float2(R[c].x + F[c].x, R[c].y + F[c].y);
+        if (x == 0) R[c].y = 0.f;
+      }
     }
   }
-  if (!HD && a.hydro) {  // B = 0: only roundoff of the paired x-row transforms would feed it
-#pragma unroll
-    for (int c = 3; c < 6; ++c) R[c] = make_float2(0.f, 0.f);
+}
+
+// Stage update of one value (RK4 and LSRK4 as in StageOp); returns the next stage state.
+__device__ __forceinline__ float2 stage_update(int op, const RkSlot& a, float2 x, float2 R, float2 s, float2 q, float2& acc) {
+  switch (op) {
+    case OP_RK4_FIRST:
+      acc = R;
+      return make_float2(fmaf(a.h, R.x, x.x), fmaf(a.h, R.y, x.y));
+    case OP_RK4_MID:  // 2 R is exact: one rounding
+      acc = make_float2(fmaf(2.f, R.x, q.x), fmaf(2.f, R.y, q.y));
+      return make_float2(fmaf(a.h, R.x, s.x), fmaf(a.h, R.y, s.y));
+    case OP_RK4_LAST:
+      return make_float2(fmaf(a.dt6, q.x + R.x, s.x), fmaf(a.dt6, q.y + R.y, s.y));
+    case OP_LS_FIRST:
+      acc = make_float2(a.dt * R.x, a.dt * R.y);
+      return make_float2(x.x + a.cb * acc.x, x.y + a.cb * acc.y);
+    case OP_LS:
+      acc = make_float2(a.ca * q.x + a.dt * R.x, a.ca * q.y + a.dt * R.y);
+      return make_float2(x.x + a.cb * acc.x, x.y + a.cb * acc.y);
+    default:  // OP_RHS
+      acc = R;
+      return x;
   }
-#pragma unroll
-  for (int c = 0; c < NF; ++c) rk_apply<OP>(rs, c * fs + i, xv[c], R[c]);
 }
 
 }  // namespace mhdgb

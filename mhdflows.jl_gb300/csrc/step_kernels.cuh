@@ -6,35 +6,82 @@
 
 namespace mhdgb {
 
-// grid (ceil(kx / blockDim.x), k2, k2): one thread per retained mode, no index division.
+// Streaming right-hand side and Runge-Kutta stage update: one thread per pair of neighbouring
+// modes of a compact field (16-byte accesses) and field triple (blockIdx.y: u, B), blockIdx.z the
+// instance.  Bound by HBM: 33.5 arrays of a field per RK4 launch on average, 105 us at 256^3
+// (6.3 TB/s) and 767 us at 512^3.  One thread per mode for all six fields took 131 and 1004 us, bound by
+// instruction issue: 76 M warp instructions at 256^3 against 34 M here, most of them the IEEE
+// divisions of R/6 and R/3 (now one multiplication by dt/6 in the last stage) and the products' scale
+// applied plane by plane.  Triples as separate blocks keep a thread at 8 to 14 loads (80 registers).
 // HD: the hydrodynamic form (three fields, five product planes; B is neither read nor written).
-template <int OP, bool FORCED, bool VPEN, bool HD = false>
-__global__ void __launch_bounds__(256) rk_epilogue_kernel(RkArgs a, Geom geo, BatchRef br) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= geo.kx) return;
-  const int inst = blockIdx.z / geo.k2;
-  if (inst >= *br.count) return;
-  const int slot = br.list[inst];
-  const int jy = blockIdx.y, jz = blockIdx.z - inst * geo.k2;
-  const long long fs = a.fs;
-  const long long i = ((long long)jz * geo.k2 + jy) * geo.kxp + x;
-  const float2* prod = a.prod + slot * a.prodI;
-  const float kxv = geo.kscale * (float)x;
-  const float kyv = geo.kscale * (float)signed_of_kept(geo, jy);
-  const float kzv = geo.kscale * (float)signed_of_kept(geo, jz);
-  float2 p[8];
+constexpr int kStageThreads = 128;
+template <int OP, bool GENERAL, bool HD>
+__global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo, BatchRef br) {
+  const unsigned int i = 2u * (blockIdx.x * kStageThreads + threadIdx.x);
+  if ((int)blockIdx.z >= *br.count) return;
+  const int slot = br.list[blockIdx.z];
+  const unsigned int row = i / (unsigned int)geo.kxp;  // a compact field has fewer than 2^32 elements
+  const int x = (int)(i - row * (unsigned int)geo.kxp), jz = (int)(row / (unsigned int)geo.k2);
+  const int jy = (int)(row - (unsigned int)jz * (unsigned int)geo.k2);
+  if (jz >= geo.k2 || x >= geo.kx) return;
+  const int t = blockIdx.y;
+  const long long so = slot * a.stI + 3 * t * a.fs + i;
+  const float2* X = a.X + so;
+  const float2* prod = a.prod + slot * a.prodI + i;
+  const int npl = t ? 3 : 5;
+  constexpr bool rd_sol = OP == OP_RK4_MID || OP == OP_RK4_LAST, rd_acc = rd_sol || OP == OP_LS;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 pl[5], pn[3], xv[3], s4[3], q4[3];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) p[q] = (HD && q >= 5) ? make_float2(0.f, 0.f) : cscale(__ldcs(prod + q * fs + i), a.pscale);
-  const float2 dxz = p[0], dyz = p[1], txy = p[2], txz = p[3], tyz = p[4];
-  const float2 axy = p[5], axz = p[6], ayz = p[7];
-  ModeSums m;
-  m.Vx = make_float2(kxv * dxz.x + kyv * txy.x + kzv * txz.x, kxv * dxz.y + kyv * txy.y + kzv * txz.y);
-  m.Vy = make_float2(kxv * txy.x + kyv * dyz.x + kzv * tyz.x, kxv * txy.y + kyv * dyz.y + kzv * tyz.y);
-  m.Vz = make_float2(kxv * txz.x + kyv * tyz.x, kxv * txz.y + kyv * tyz.y);
-  m.Wx = make_float2(kyv * axy.x + kzv * axz.x, kyv * axy.y + kzv * axz.y);
-  m.Wy = make_float2(kzv * ayz.x - kxv * axy.x, kzv * ayz.y - kxv * axy.y);
-  m.Wz = make_float2(-(kxv * axz.x + kyv * ayz.x), -(kxv * axz.y + kyv * ayz.y));
-  finish_mode<OP, FORCED, VPEN, HD>(a, geo, slot, jz, jy, x, i, kxv, kyv, kzv, m, prod);
+  for (int q = 0; q < 5; ++q)
+    pl[q] = q < npl ? __ldcs(reinterpret_cast<const float4*>(prod + (5 * t + q) * a.fs)) : zero4;
+  const RkSlot rs0{a.sol + so, a.acc + so, a.xn + so, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    xv[c] = *reinterpret_cast<const float4*>(X + c * a.fs);
+    s4[c] = rd_sol ? *reinterpret_cast<const float4*>(rs0.sol + c * a.fs) : zero4;
+    q4[c] = rd_acc ? *reinterpret_cast<const float4*>(rs0.acc + c * a.fs) : zero4;
+    if constexpr (GENERAL) {
+      const int pp = HD ? (c == 0 ? 6 : c == 1 ? 7 : 5) : 8 + 3 * t + c;
+      pn[c] = a.vpen ? __ldcs(reinterpret_cast<const float4*>(prod + pp * a.fs)) : zero4;
+    }
+  }
+  const SlotParams sp = a.sp[slot];
+  const RkSlot rs{rs0.sol, rs0.acc, rs0.xn, a.hf * sp.dt, sp.dt, sp.dt / 6.f, a.ca, a.cb};
+  // the kx = 0 plane diffuses its Hermitian part, H[f][kz'][ky'] (written before X is updated)
+  const long long hpl = (long long)geo.k2 * geo.k2;
+  const float2* H = a.H + slot * a.hI + 3 * t * hpl + jz * geo.k2 + jy;
+  float2 nx[3][2], ac[3][2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    auto half = [&](const float4& v) { return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y); };
+    const int xh = x + h;
+    float2 p[5], pen[3], d[3], R[3];
+#pragma unroll
+    for (int q = 0; q < 5; ++q) p[q] = half(pl[q]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      d[c] = half(xv[c]);
+      if (xh == 0) d[c] = H[c * hpl];
+      if constexpr (GENERAL) pen[c] = half(pn[c]);
+    }
+    const float kxv = geo.kscale * (float)xh;
+    const float kyv = geo.kscale * (float)signed_of_kept(geo, jy);
+    const float kzv = geo.kscale * (float)signed_of_kept(geo, jz);
+    triple_rhs<GENERAL, HD>(a, geo, sp, slot, t, xh, jy, jz, kxv, kyv, kzv, d, p, pen, R);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nx[c][h] = stage_update(OP, rs, half(xv[c]), R[c], half(s4[c]), half(q4[c]), ac[c][h]);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const float4 n4 = make_float4(nx[c][0].x, nx[c][0].y, nx[c][1].x, nx[c][1].y);
+    if constexpr (OP == OP_RK4_LAST) {
+      *reinterpret_cast<float4*>(rs.sol + c * a.fs) = n4;
+    } else {
+      *reinterpret_cast<float4*>(rs.acc + c * a.fs) = make_float4(ac[c][0].x, ac[c][0].y, ac[c][1].x, ac[c][1].y);
+      if constexpr (OP != OP_RHS) *reinterpret_cast<float4*>(rs.xn + c * a.fs) = n4;
+    }
+  }
 }
 
 // On-device getCFL! (src/integrator.jl:158-198 of MHDFlows.jl) after a step of every active
