@@ -96,6 +96,9 @@ Geom make_geom(int n, double L) {
   g.kxp = (g.kx + 3) / 4 * 4;
   g.k2 = g.kp + g.kn;
   g.kscale = (float)(2.0 * M_PI / L);
+  g.planar = 0;
+  g.k2p = (g.k2 + 3) / 4 * 4;
+  g.fs = (long long)g.k2 * g.k2 * g.kxp;
   return g;
 }
 
@@ -167,6 +170,18 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
   }();
   return fn;
+}
+
+// 4-D tensor map over the R planes [inst][slot kx][z][y] of the plane passes: boxes of one slot's kx
+// modes x 16 y (128-byte rows, 128-byte swizzle)
+bool make_plane_tmap(CUtensorMap* m, void* base, cuuint64_t n, cuuint64_t planes, cuuint64_t insts, cuuint64_t inst_bytes,
+                     cuuint32_t kx) {
+  auto enc = tmap_encoder();
+  if (!enc) return false;
+  const cuuint64_t dims[4] = {n, n, planes, insts}, strides[3] = {n * 8, n * n * 8, inst_bytes};
+  const cuuint32_t box[4] = {16, 1, kx, 1}, es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // 5-D tensor map over 8-byte elements (complex float pairs), no swizzle, zero fill out of range
@@ -316,6 +331,7 @@ struct mhd_problem {
   bool divcorr = false;
   // TMA sources of the column passes (used when a TMA-fed variant is selected) and the device
   // word a timed-out tile wait is recorded in
+  TmaPass tm_plane;  // plane order: the R planes
   TmaPass tm_zinv_sol, tm_zinv_xs, tm_yinv, tm_yfwd, tm_zfwd;
   int* derr = nullptr;
   bool cfl = false;
@@ -376,6 +392,7 @@ struct mhd_problem {
   cudaGraphExec_t graph_diag = nullptr;
   // profiling
   bool profiling = false;
+  bool tuning = false;  // a right-hand side also runs the fused inverse pass of its (unchanged) state
   struct Rec { int cls; cudaEvent_t a, b; };
   std::vector<Rec> recs;
   std::vector<cudaEvent_t> pool;
@@ -488,7 +505,7 @@ struct mhd_problem {
   int x_fused(BatchRef br, unsigned int* vmax) {
     // the six field rows of a physical row are contiguous (slot stride == kxp)
     const VpRef vp{vchi, vwall, sz.phys};
-    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, SLK(), g.kxp, sz.rowbuf, br, cap, vmax, vp, stream); });
+    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, row_stride(), row_slot(), sz.rowbuf, br, cap, vmax, vp, stream, &tm_plane); });
   }
   int y_forward(int nf, BatchRef br) {
     ColArgs a{rowbuf, colbuf, (long long)g.kxp, BZ(), SLK(), (long long)g.kxp, AZ(), SLK(), sz.rowbuf, sz.colbuf};
@@ -506,6 +523,23 @@ struct mhd_problem {
     a.hoI = FS();
     return launch(KC_ZFWD, [&] { ops->col(KC_ZFWD, a, g, g.k2, nf, br, cap, stream, &tm_zfwd); });
   }
+  // ---- plane order (small grids): planes R[slot][kx][z][y] in rowbuf, products in colbuf
+  // compact fields (src + slot*sI, nf fields at stride FS) -> R planes 0..nf-1
+  int plane_inverse(const float2* src, long long sI, int nf, BatchRef br) {
+    // where the stage update is fused with the inverse pass, that launch is the tuned z_inverse class
+    const int cls = plane_fused(g.n) ? KC_OTHER : KC_ZINV;
+    const PlaneArgs a{src, rowbuf, sI, sz.rowbuf, FS(), nullptr, nullptr, 0, 0, 0};
+    return launch(cls, [&] { ops->plane_inverse(a, g, nf, br, cap, stream); });
+  }
+  // R planes 0..nf-1 -> compact planes at dst + slot*dI
+  // hx: as z_forward's
+  int plane_forward(float2* dst, long long dI, int nf, BatchRef br, const float2* hx = nullptr) {
+    const PlaneArgs a{rowbuf, dst, sz.rowbuf, dI, FS(), hx, aux, ST(), FS(), nfields()};
+    return launch(KC_ZFWD, [&] { ops->plane_forward(a, g, nf, br, cap, stream); });
+  }
+  // strides of the physical rows in rowbuf
+  long long row_stride() const { return g.planar ? 1 : SLK(); }
+  long long row_slot() const { return g.planar ? (long long)g.kx * g.n * g.n : g.kxp; }
   // Stage epilogue: RHS from the 8 compact product planes (in rowbuf; 14 with the VP penalty
   // fields) and the stage state X.
   RkArgs rk_args(const float2* X, float2* xn, int op, float hf, float ca, float cb, int stage) const {
@@ -540,8 +574,12 @@ struct mhd_problem {
   // xn: where the stage update writes (the next stage state, or sol; it may be X itself, so the
   // Hermitian part of X's kx = 0 plane was copied out into aux by the z_forward before it)
   int epilogue(const float2* X, float2* xn, int op, float hf, float ca, float cb, BatchRef br, int stage) {
-    const RkArgs a = rk_args(X, xn, op, hf, ca, cb, stage);
-    const dim3 grid((unsigned)((FS() / 2 + kStageThreads - 1) / kStageThreads), hd_form() ? 1 : 2, cap);
+    RkArgs a = rk_args(X, xn, op, hf, ca, cb, stage);
+    if (g.planar) {
+      a.prod = colbuf;
+      a.prodI = sz.colbuf;
+    }
+    const dim3 grid((unsigned)((field_elems(g) / 2 + kStageThreads - 1) / kStageThreads), hd_form() ? 1 : 2, cap);
     return launch(KC_RKEPI, [&] {
       if (hd_form()) launch_epilogue<true, true>(op, grid, a, br);
       else if (a.vpen || a.forced) launch_epilogue<true, false>(op, grid, a, br);
@@ -562,14 +600,28 @@ struct mhd_problem {
   }
   // DivVCorrection! / DivBCorrection! of the slots in br (mask: 1 u, 2 B)
   int div_correct(BatchRef br, int ninst, int mask) {
-    const int bx = g.kx <= 256 ? (g.kx + 31) / 32 * 32 : 256;
-    const dim3 grid((g.kx + bx - 1) / bx, g.k2, g.k2 * ninst);
-    return launch(KC_OTHER, [&] { div_correct_kernel<<<grid, bx, 0, stream>>>(sol, g, FS(), ST(), br, mask); });
+    const dim3 grid((unsigned)((field_elems(g) + 255) / 256), ninst);
+    return launch(KC_OTHER, [&] { div_correct_kernel<<<grid, 256, 0, stream>>>(sol, g, FS(), ST(), br, mask); });
   }
   // stage: right-hand-side evaluation within the step (7 outside a step)
   int rhs(const float2* X, float2* xn, int op, float hf, float ca, float cb, BatchRef br, int stage, bool record = false) {
     int rc;
     const int nin = hd_form() ? 3 : 6, nout = hd_form() ? (p.vp ? 8 : 5) : ns;
+    if (g.planar) {
+      // a fused stage before this one left the planes of X in rowbuf
+      const bool fused = plane_fused(g.n);
+      if (!fused || stage == 0 || stage == 7)
+        if ((rc = plane_inverse(X, ST(), nin, br))) return rc;
+      if ((rc = x_fused(br, (record && cfl) ? dvmax : nullptr))) return rc;
+      if ((rc = plane_forward(colbuf, sz.colbuf, nout, br, fused ? nullptr : X))) return rc;
+      if (!fused) return epilogue(X, xn, op, hf, ca, cb, br, stage);
+      const bool inv = (op != OP_RHS || tuning) && !record;
+      RkArgs a = rk_args(X, xn, op, hf, ca, cb, stage);
+      a.prod = colbuf;
+      a.prodI = sz.colbuf;
+      const PlaneArgs pa{nullptr, rowbuf, 0, sz.rowbuf, FS(), nullptr, nullptr, 0, 0, 0};
+      return launch(inv ? KC_ZINV : KC_RKEPI, [&] { ops->plane_stage(a, pa, g, nin, inv, br, cap, stream); });
+    }
     if ((rc = z_inverse(X, ST(), nin, br))) return rc;
     if ((rc = y_inverse(nin, br))) return rc;
     if ((rc = x_fused(br, (record && cfl) ? dvmax : nullptr))) return rc;
@@ -661,7 +713,7 @@ struct mhd_problem {
     int base[kTunedClasses];
     std::memcpy(base, ops->sel, sizeof(base));
     int rc = MHD_OK;
-    profiling = true;
+    profiling = tuning = true;
     for (int sweep = 0; sweep < 2 && rc == MHD_OK; ++sweep)
       for (int r = 0; r < maxv && rc == MHD_OK; ++r) {
         for (int c = 0; c < kTunedClasses; ++c) ops->sel[c] = ops->variant_ok(c, r) ? r : base[c];
@@ -678,7 +730,7 @@ struct mhd_problem {
           if (ops->variant_ok(c, r) && prof_launches[c] > 0)
             best[c][r] = std::min(best[c][r], prof_ms[c] / prof_launches[c]);
       }
-    profiling = false;
+    profiling = tuning = false;
     for (auto& rec : recs) { pool.push_back(rec.a); pool.push_back(rec.b); }
     recs.clear();
     for (int c = 0; c < KC_COUNT; ++c) { prof_launches[c] = 0; prof_ms[c] = 0; }
@@ -779,18 +831,23 @@ struct mhd_problem {
   int inverse_field(const float2* src, long long sI, int slot, float scale = -1.f) {
     int rc;
     const BatchRef br = slot_ref(slot);
-    if ((rc = z_inverse(src, sI, 1, br))) return rc;
-    if ((rc = y_inverse(1, br))) return rc;
+    if (g.planar) {
+      if ((rc = plane_inverse(src, sI, 1, br))) return rc;
+    } else {
+      if ((rc = z_inverse(src, sI, 1, br))) return rc;
+      if ((rc = y_inverse(1, br))) return rc;
+    }
     float2* rb = rowbuf + slot * sz.rowbuf;
     const float sc = scale < 0.f ? (float)(1.0 / ((double)g.n * g.n * g.n)) : scale;
-    return launch(KC_OTHER, [&] { ops->x_c2r(rb, phys, g, SLK(), sc, stream); });
+    return launch(KC_OTHER, [&] { ops->x_c2r(rb, phys, g, row_stride(), sc, stream); });
   }
   // One field of one slot: physical staging -> compact (dst + slot*dI), unnormalised forward.
   int forward_field(float2* dst, long long dI, int slot) {
     int rc;
     const BatchRef br = slot_ref(slot);
     float2* rb = rowbuf + slot * sz.rowbuf;
-    if ((rc = launch(KC_OTHER, [&] { ops->x_r2c(phys, rb, g, SLK(), stream); }))) return rc;
+    if ((rc = launch(KC_OTHER, [&] { ops->x_r2c(phys, rb, g, row_stride(), stream); }))) return rc;
+    if (g.planar) return plane_forward(dst, dI, 1, br);
     if ((rc = y_forward(1, br))) return rc;
     return z_forward(dst, dI, 1, br);
   }
@@ -799,6 +856,11 @@ struct mhd_problem {
   // named; rows = the transformed axis).  A map that cannot be encoded leaves the pass on the
   // cp.async kernels.
   void build_tma() {
+    if (g.planar) {
+      tm_plane.ok = make_plane_tmap(&tm_plane.map, rowbuf, g.n, (cuuint64_t)ns * g.kx, cap, (cuuint64_t)sz.rowbuf * sizeof(float2), g.kx);
+      tm_plane.err = derr;
+      return;
+    }
     const cuuint64_t E = sizeof(float2), kxp = g.kxp, k2 = g.k2, n = g.n, C = cap;
     const cuuint32_t kp = g.kp, rb = g.n <= 256 ? g.n : 256;
     auto set = [&](TmaPass& t, void* base, const cuuint64_t (&d)[5], const cuuint64_t (&st)[4],
@@ -911,6 +973,9 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   h->ops->prec = params->precision;
   h->ops->vp_capable = params->vp != 0;
   h->ops->hd = h->hd_form() ? 1 : 0;
+  h->ops->planar = !h->ops->pv.empty() && params->precision == MHD_PREC_FP32;
+  h->g.planar = h->ops->planar ? 1 : 0;
+  h->ops->batch = cap > 1;
   if ((rc = h->ops->setup(h->g))) return rc;
   if (params->vp && (rc = h->ops->set_vp(1))) return rc;  // mask only until walls are set
   {

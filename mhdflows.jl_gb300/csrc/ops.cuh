@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "passes.cuh"
+#include "plane_kernels.cuh"
 #include "tc5_rows.cuh"
 #include "tc_rows.cuh"
 
@@ -41,13 +42,19 @@ struct TmaPass {
 };
 using C2RFn = void (*)(const float2*, float*, Geom, long long, float, const float2*);
 using R2CFn = void (*)(const float*, float2*, Geom, long long, const float2*);
+using PlaneFwdFn = void (*)(PlaneArgs, Geom, BatchRef, const float2*);
+using PlaneInvFn = void (*)(PlaneArgs, BatchRef, const float2*);
+using PlaneStageFn = void (*)(RkArgs, PlaneArgs, Geom, BatchRef, int, const float2*);
+using XPlaneFn = void (*)(CUtensorMap, int*, BatchRef, const float2*, const float2*, unsigned int*, VpRef);
 
 struct XVariant {
   std::string name;
   XFn fn = nullptr;
+  XPlaneFn tile_fn = nullptr;         // tiles in plane order by TMA (fn unused then)
   int threads = 0, rpg = 1, groups = 1;
   int (*group_words)(int) = nullptr;  // shared-memory words of one row group for a padded row length
   size_t tw = 0, twr = 0;             // offsets of the plan's twiddles and of its reverse's
+  size_t tile_smem = 0;
   size_t smem = 0;
   int ctas = 0;                       // resident CTAs on the device (0: does not fit)
   // precision form: 0 FP32, 1 split FP16 tensor cores, 2 split BF16 tensor cores; the split
@@ -61,6 +68,7 @@ struct XVariant {
   int (*build_table)(uint32_t* table) = nullptr;
   uint32_t* table = nullptr;
   int err_word = -1;  // index of a device error word in the table (bounded waits), -1: none
+  bool plane = false;  // rows in plane order
   bool max_carveout = false;  // ask for the largest shared-memory carveout of the L1 array
 };
 
@@ -74,6 +82,20 @@ struct ColVariant {
   int ctas_inv = 0, ctas_fwd = 0;
 };
 
+// Plane passes of a small grid (plane_kernels.cuh): one plan and block size; the stage kernel in
+// its plain form, with penalty planes or forcing, and the hydrodynamic form.
+struct PlaneVariant {
+  std::string name;
+  PlaneFwdFn fwd = nullptr;
+  PlaneInvFn inv = nullptr;
+  PlaneStageFn stage = nullptr, stage_gen = nullptr, stage_hd = nullptr;
+  int threads = 0;
+  size_t tw = 0;
+  size_t smem = 0;
+  int ctas_fwd = 0, ctas_inv = 0;
+  int pref = 0;  // default of: bit 0 inverse, bit 1 forward of a single problem; bits 2, 3 of a batch
+};
+
 class OpsBase {
  public:
   virtual ~OpsBase();
@@ -84,7 +106,15 @@ class OpsBase {
   void col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, int cap, cudaStream_t s,
            const TmaPass* tp = nullptr) const;
   void x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride, BatchRef br,
-               int cap, unsigned int* vmax, VpRef vp, cudaStream_t s) const;
+               int cap, unsigned int* vmax, VpRef vp, cudaStream_t s, const TmaPass* tp = nullptr) const;
+  // plane passes: forward transforms of nslots planes per kx mode; stage update (a.op) of nf
+  // fields and, with inv, their inverse transforms.  cap as in col.
+  void plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, int cap, cudaStream_t s) const;
+  void plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, int cap, cudaStream_t s) const;
+  void plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, int nf, bool inv, BatchRef br, int cap,
+                   cudaStream_t s) const;
+  // x rows in plane order by TMA tiles, map over the R planes (a variant that reads the planes directly
+  // when the map could not be encoded)
   void x_c2r(const float2* src, float* dst, const Geom& g, long long srow, float scale, cudaStream_t s) const;
   void x_r2c(const float* src, float2* dst, const Geom& g, long long drow, cudaStream_t s) const;
   // a bounded device wait of the selected x-row kernel that ran out (its table's error word);
@@ -101,6 +131,11 @@ class OpsBase {
   int set_vp(int mode);
   std::vector<XVariant> xv;
   std::vector<ColVariant> cv;
+  // plane order (set before setup): the column classes are the plane passes, y_inverse and
+  // y_forward being part of z_inverse's and z_forward's launches
+  bool planar = false;
+  bool batch = false;  // capacity above 1 (set before setup): picks the default plane variants
+  std::vector<PlaneVariant> pv;
   int sel[kTunedClasses] = {0, 0, 0, 0, 0};  // selected variant of each tuned class
   int variant_count(int cls) const;
   bool variant_ok(int cls, int i) const;
@@ -110,8 +145,8 @@ class OpsBase {
 
  protected:
   // plain row transforms (staging of set_physical / get_physical / diagnostics)
-  C2RFn c2r = nullptr;
-  R2CFn r2c = nullptr;
+  C2RFn c2r = nullptr, c2r_plane = nullptr;
+  R2CFn r2c = nullptr, r2c_plane = nullptr;
   int rows = 1, row_threads = 0;
   size_t row_smem = 0, row_tw = 0;
   std::vector<float2> tw_host;
@@ -170,14 +205,15 @@ class Ops : public OpsBase {
     add_x_form<R, GROUPS, NTI, NTF, MINB, false>();
   }
   // DIRECT: field rows loaded from global memory into registers, no staging copy ("/d")
-  template <class R, int GROUPS, int NTI, int NTF, int MINB, bool DIRECT>
+  template <class R, int GROUPS, int NTI, int NTF, int MINB, bool DIRECT, bool PLANE = false>
   void add_x_form() {
     constexpr int NTS = NTI > NTF ? NTI : NTF;
     using XC = XCfg<R, NTS, DIRECT>;
     XVariant v;
-    v.name = "x:" + plan_name<R>() + "/nt" + std::to_string(NTI) + std::to_string(NTF) + "/c" +
-             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (DIRECT ? "/d" : "");
-    v.fn = x_fused_kernel<R, GROUPS, NTI, NTF, MINB, 0, false, DIRECT>;
+    v.plane = PLANE;
+    v.name = std::string(PLANE ? "xplane:" : "x:") + plan_name<R>() + "/nt" + std::to_string(NTI) + std::to_string(NTF) + "/c" +
+             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (DIRECT && !PLANE ? "/d" : "");
+    v.fn = x_fused_kernel<R, GROUPS, NTI, NTF, MINB, 0, false, DIRECT, PLANE>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -187,20 +223,40 @@ class Ops : public OpsBase {
     xv.push_back(v);
   }
 
+  // x rows in plane order by TMA tiles, NBUF tiles in flight per CTA
+  template <class R, int NBUF, int MINB, int VPM = 0, bool HDX = false>
+  void add_x_tile() {
+    using XC = XPlaneCfg<R, NBUF, VPM, HDX>;
+    XVariant v;
+    v.name = std::string(HDX ? "xtilehd" : "xtile") + (VPM ? "vp" + std::to_string(VPM) : "") + ":" + plan_name<R>() + "/q" +
+             std::to_string(NBUF) + "/b" + std::to_string(MINB);
+    v.tile_fn = x_plane_kernel<R, NBUF, MINB, VPM, HDX>;
+    v.threads = XC::THREADS;
+    v.rpg = XC::ROWS;
+    v.tile_smem = XC::SMEM;
+    v.tw = twiddles<R>();
+    v.twr = twiddles<typename Reverse<R>::type>();
+    v.vp = VPM;
+    v.hd = HDX ? 1 : 0;
+    v.plane = true;
+    xv.push_back(v);
+  }
+
   // x rows with the volume-penalisation pairs: the mask-only and the mask-and-walls forms of a
   // plan, one forward transform per exchange round
-  template <class R, int GROUPS, int NTI, int MINB>
+  template <class R, int GROUPS, int NTI, int MINB, bool PLANE = false>
   void add_x_vp() {
-    add_x_vp_one<R, GROUPS, NTI, MINB, 1>();
-    add_x_vp_one<R, GROUPS, NTI, MINB, 2>();
+    add_x_vp_one<R, GROUPS, NTI, MINB, 1, PLANE>();
+    add_x_vp_one<R, GROUPS, NTI, MINB, 2, PLANE>();
   }
-  template <class R, int GROUPS, int NTI, int MINB, int VPM>
+  template <class R, int GROUPS, int NTI, int MINB, int VPM, bool PLANE>
   void add_x_vp_one() {
-    using XC = XCfg<R, NTI>;
+    using XC = XCfg<R, NTI, PLANE>;
     XVariant v;
+    v.plane = PLANE;
     v.name = "xvp" + std::to_string(VPM) + ":" + plan_name<R>() + "/nt" + std::to_string(NTI) + "1/c" +
              std::to_string(GROUPS) + "/b" + std::to_string(MINB);
-    v.fn = x_fused_kernel<R, GROUPS, NTI, 1, MINB, VPM>;
+    v.fn = x_fused_kernel<R, GROUPS, NTI, 1, MINB, VPM, false, PLANE, PLANE>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -213,13 +269,14 @@ class Ops : public OpsBase {
 
   // x rows of the hydrodynamic form (one transform per exchange round); VPM > 0 adds the
   // velocity penalty fields (VP on hydrodynamics)
-  template <class R, int GROUPS, int MINB, int VPM = 0>
+  template <class R, int GROUPS, int MINB, int VPM = 0, bool PLANE = false>
   void add_x_hd() {
-    using XC = XCfg<R, 1>;
+    using XC = XCfg<R, 1, PLANE>;
     XVariant v;
+    v.plane = PLANE;
     v.name = std::string(VPM ? "xhdvp" + std::to_string(VPM) : "xhd") + ":" + plan_name<R>() + "/nt11/c" +
              std::to_string(GROUPS) + "/b" + std::to_string(MINB);
-    v.fn = x_fused_kernel<R, GROUPS, 1, 1, MINB, VPM, true>;
+    v.fn = x_fused_kernel<R, GROUPS, 1, 1, MINB, VPM, true, PLANE, PLANE>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -231,10 +288,30 @@ class Ops : public OpsBase {
     xv.push_back(v);
   }
   // both penalisation forms (mask only, mask and walls) of the hydrodynamic x rows
-  template <class R, int GROUPS, int MINB>
+  template <class R, int GROUPS, int MINB, bool PLANE = false>
   void add_x_hdvp() {
-    add_x_hd<R, GROUPS, MINB, 1>();
-    add_x_hd<R, GROUPS, MINB, 2>();
+    add_x_hd<R, GROUPS, MINB, 1, PLANE>();
+    add_x_hd<R, GROUPS, MINB, 2, PLANE>();
+  }
+
+  // plane passes with T threads per plane, and the plain row kernels in plane order
+  template <class P, int T, int MINB>
+  void add_plane(int pref = 15) {
+    using C = PlaneCfg<P, T, MINB>;
+    PlaneVariant v;
+    v.name = "plane:" + plan_name<P>() + "/t" + std::to_string(T) + "/b" + std::to_string(MINB);
+    v.fwd = plane_forward_kernel<C>;
+    v.inv = plane_inverse_kernel<C>;
+    if constexpr (plane_fused(N)) {
+      v.stage = plane_stage_kernel<C, false, false>;
+      v.stage_gen = plane_stage_kernel<C, true, false>;
+      v.stage_hd = plane_stage_kernel<C, true, true>;
+    }
+    v.threads = T;
+    v.smem = C::SMEM;
+    v.tw = twiddles<P>();
+    v.pref = pref;
+    pv.push_back(v);
   }
 
   // x rows on the tensor cores (split FP16 or BF16 operands), GROUPS warps (rows) per CTA
@@ -310,6 +387,10 @@ class Ops : public OpsBase {
   void set_rows() {
     c2r = x_c2r_kernel<R, ROWS>;
     r2c = x_r2c_kernel<R, ROWS>;
+    if constexpr (N <= kPlaneMax) {
+      c2r_plane = x_c2r_kernel<R, ROWS, true>;
+      r2c_plane = x_r2c_kernel<R, ROWS, true>;
+    }
     rows = ROWS;
     row_threads = ROWS * R::G;
     row_smem = sizeof(float2) * (size_t)RowCfg<R>::TS * ROWS;

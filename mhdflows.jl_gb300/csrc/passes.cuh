@@ -22,7 +22,34 @@ struct Geom {
   int kn;     // kept negative full-axis modes
   int k2;     // kp + kn
   float kscale;  // 2*pi/L
+  int planar;    // 1: compact fields in plane order [kx][kz'][ky'] (plane_kernels.cuh)
+  int k2p;       // plane order: padded ky' row length
+  long long fs;  // compact field stride
 };
+
+// Offset of a mode inside a compact field, and the mode at an offset (false: a padding element).
+__host__ __device__ inline long long mode_off(const Geom& g, int x, int jy, int jz) {
+  return g.planar ? ((long long)x * g.k2 + jz) * g.k2p + jy : ((long long)jz * g.k2 + jy) * g.kxp + x;
+}
+__host__ __device__ inline bool mode_at(const Geom& g, long long i, int& x, int& jy, int& jz) {
+  const unsigned int q = (unsigned int)i;  // a compact field has fewer than 2^32 elements
+  if (g.planar) {
+    const unsigned int r = q / (unsigned int)g.k2p;
+    jy = (int)(q - r * (unsigned int)g.k2p);
+    x = (int)(r / (unsigned int)g.k2);
+    jz = (int)(r - (unsigned int)x * (unsigned int)g.k2);
+    return jy < g.k2;
+  }
+  const unsigned int r = q / (unsigned int)g.kxp;
+  x = (int)(q - r * (unsigned int)g.kxp);
+  jz = (int)(r / (unsigned int)g.k2);
+  jy = (int)(r - (unsigned int)jz * (unsigned int)g.k2);
+  return x < g.kx;
+}
+// elements of a compact field, padding included
+__host__ __device__ inline long long field_elems(const Geom& g) {
+  return g.planar ? (long long)g.kx * g.k2 * g.k2p : (long long)g.k2 * g.k2 * g.kxp;
+}
 
 __host__ __device__ inline int kept_of_freq(const Geom& g, int f) {
   return f < g.kp ? f : (f >= g.n - g.kn ? f - g.n + g.k2 : -1);
@@ -514,15 +541,14 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
 // x rows: Hermitian two-for-one helpers.
 // ------------------------------------------------------------------------------------------
 // Input of an inverse (c2r) transform of two half-spectrum rows f1, f2 with KX kept modes
-// (plain loads: the rows may live in global or in shared memory):
+// (f(n): mode n of a row, which may live in global or in shared memory):
 // z[n] = F1[n] + i F2[n] with F[n-n] = conj(F[n]); the kx = 0 imaginary parts are dropped,
 // which is what a c2r transform does with a non-Hermitian kx = 0 plane.  Elements whose index
 // lies in the alias band for every lane are compile-time zeros, so the first stage of the
 // transform is pruned by constant folding.
 // ZB: the second field is zero (f2 is not read).
-template <class P, int KX, bool ZB = false>
-__device__ __forceinline__ void load_herm_pair(float2 (&v)[P::V], const float2* __restrict__ f1,
-                                               const float2* __restrict__ f2, int g) {
+template <class P, int KX, bool ZB = false, class F1, class F2>
+__device__ __forceinline__ void load_herm_pair(float2 (&v)[P::V], F1 f1, F2 f2, int g) {
 #pragma unroll
   for (int d = 0; d < P::DI; ++d)
 #pragma unroll
@@ -532,29 +558,36 @@ __device__ __forceinline__ void load_herm_pair(float2 (&v)[P::V], const float2* 
       if (nmin < KX || nmin + P::G - 1 > P::N - KX) {  // some lane holds a kept mode
         const int n = g + nmin;
         if (n < KX) {
-          float2 a = f1[n], b = ZB ? make_float2(0.f, 0.f) : f2[n];
+          float2 a = f1(n), b = ZB ? make_float2(0.f, 0.f) : f2(n);
           if (n == 0) { a.y = 0.f; b.y = 0.f; }
           z = make_float2(a.x - b.y, a.y + b.x);
         } else if (n > P::N - KX) {
           const int m = P::N - n;
-          float2 a = f1[m], b = ZB ? make_float2(0.f, 0.f) : f2[m];
+          float2 a = f1(m), b = ZB ? make_float2(0.f, 0.f) : f2(m);
           z = make_float2(a.x + b.y, b.x - a.y);
         }
       }
       v[d * P::R0 + n0] = z;
     }
 }
+// a row in memory, XS between kx modes (1 for contiguous rows, n^2 in plane order)
+template <int XS>
+struct RowRead {
+  const float2* p;
+  __device__ __forceinline__ float2 operator()(int n) const { return p[n * XS]; }
+};
 
 // Split Z = FFT(pa + i pb) into the half spectra of pa and pb for k < kx and store them.
-// sb holds Z[k] for every needed k (k < kx and k > n - kx).
+// sb holds Z[k] for every needed k (k < kx and k > n - kx).  XS as RowRead.
+template <int XS = 1>
 __device__ __forceinline__ void store_split_pair(const float2* sb, int n, int kx, int g, int G,
                                                  float2* outa, float2* outb) {
   for (int k = g; k < kx; k += G) {
     const float2 z = sb[k];
     const float2 zc = cconj(sb[(n - k) % n]);
     const float2 s = cadd(z, zc), df = csub(z, zc);
-    outa[k] = make_float2(0.5f * s.x, 0.5f * s.y);
-    outb[k] = make_float2(0.5f * df.y, -0.5f * df.x);
+    outa[k * XS] = make_float2(0.5f * s.x, 0.5f * s.y);
+    outb[k * XS] = make_float2(0.5f * df.y, -0.5f * df.x);
   }
 }
 
@@ -563,10 +596,10 @@ __device__ __forceinline__ void store_split_pair(const float2* sb, int n, int kx
 // register (m % DF)*RF + m / DF of lane g holds Z[g + G m], and Z[N - g - G m] sits in lane
 // (G - g) % G at index V-1-m (g > 0) or in lane 0 itself at index (V-m) % V (g = 0): one
 // shuffle per needed output, no shared memory.  Outputs of every lane past the kept band are
-// never read, so the last stage of the transform is pruned as dead code.
-template <class P, int KX>
-__device__ __forceinline__ void store_split_shfl(const float2 (&v)[P::V], int g, int rowbase, float2* outa,
-                                                 float2* outb) {
+// never read, so the last stage of the transform is pruned as dead code.  put(k, a, b) takes
+// mode k of the two half spectra.
+template <class P, int KX, class Put>
+__device__ __forceinline__ void split_shfl(const float2 (&v)[P::V], int g, int rowbase, Put put) {
   constexpr int G = P::G, V = P::V, DF = P::DF, RF = P::RF;
   static_assert(G <= 32, "the shuffle split needs the row inside one warp");
   const int partner = rowbase + (G - g) % G;
@@ -584,8 +617,7 @@ __device__ __forceinline__ void store_split_shfl(const float2 (&v)[P::V], int g,
     if (k < KX) {
       const float2 zc = cconj(p);
       const float2 s = cadd(z, zc), df = csub(z, zc);
-      outa[k] = make_float2(0.5f * s.x, 0.5f * s.y);
-      outb[k] = make_float2(0.5f * df.y, -0.5f * df.x);
+      put(k, make_float2(0.5f * s.x, 0.5f * s.y), make_float2(0.5f * df.y, -0.5f * df.x));
     }
   }
 }
@@ -597,6 +629,77 @@ struct RowCfg {
   static constexpr int b = a > P::N ? a : P::N;
   static constexpr int TS = (b + 1) / 2 * 2;  // words per transform buffer (even: 16-byte aligned)
 };
+
+// Values of forward pair t at the physical points of a row: w = (first, second) product of the
+// pair, formed from the field pairs v = (ux uy | uz bx | by bz).  The MHD pairs are (Dxz, Dyz),
+// (Txy, Txz), (Tyz, Axy), (Axz, Ayz); t >= 4 the penalty pairs; the hydrodynamic form with
+// penalisation fills the spare halves (see x_fused_kernel).  chi: the mask at this thread's points;
+// wrow: the wall rows (VPM 2), component stride cs.
+template <class P, int VPM, bool HDX>
+__device__ __forceinline__ void x_pair(float2 (&w)[P::V], int t, const float2 (&v)[3][P::V], const float* chi,
+                                       const float* __restrict__ wrow, long long cs, int g) {
+  constexpr int G = P::G, V = P::V, N = P::N;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    const float ux = v[0][i].x, uy = v[0][i].y, uz = v[1][i].x;
+    const float bx = v[1][i].y, by = v[2][i].x, bz = v[2][i].y;
+    if (HDX && VPM > 0 && t >= 2) {
+      if constexpr (HDX && VPM > 0) {
+        constexpr float n3 = (float)N * (float)N * (float)N;
+        const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
+        auto wall = [&](int c) { return VPM == 2 ? n3 * __ldg(wrow + c * cs + x) : 0.f; };
+        // scaled by n^3 to the products' magnitude (n^6 times physical): a pair whose halves
+        // differ by n^3 would lose the small half to the large one's rounding in the split
+        const float c3 = n3 * chi[i];
+        if (t == 2) w[i] = make_float2(-uy * uz, c3 * (uz - wall(2)));
+        else w[i] = make_float2(c3 * (ux - wall(0)), c3 * (uy - wall(1)));
+      }
+    } else if (t >= 4) {  // penalty pair t - 4: (u x, u y), (u z, B x), (B y, B z) of the field pairs
+      if constexpr (VPM > 0) {
+        float2 f = v[t - 4][i];
+        if constexpr (VPM == 2) {  // the fields are n^3 times physical: so are the walls
+          constexpr float n3 = (float)N * (float)N * (float)N;
+          const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
+          const long long c0 = (long long)(2 * (t - 4)) * cs;
+          f.x = fmaf(-n3, __ldg(wrow + c0 + x), f.x);
+          f.y = fmaf(-n3, __ldg(wrow + c0 + cs + x), f.y);
+        }
+        w[i] = make_float2(chi[i] * f.x, chi[i] * f.y);
+      }
+    } else if (t == 0) {
+      const float tzz = bz * bz - uz * uz;
+      w[i] = make_float2((bx * bx - ux * ux) - tzz, (by * by - uy * uy) - tzz);
+    } else if (t == 1) {
+      w[i] = make_float2(bx * by - ux * uy, bx * bz - ux * uz);
+    } else if (t == 2) {
+      w[i] = make_float2(by * bz - uy * uz, ux * by - bx * uy);
+    } else {
+      w[i] = make_float2(ux * bz - bx * uz, uy * bz - by * uz);
+    }
+  }
+}
+
+// Maxima of |u_i| and |B_i| over the physical fields of one warp's rows into vm[0], vm[1] (getCFL!
+// on the last stage's fields); non-negative floats order like their bit patterns, NaN above +inf.
+template <int V>
+__device__ __forceinline__ void x_vmax(const float2 (&v)[3][V], unsigned int* vm) {
+  float mu = 0.f, mb = 0.f;
+#pragma unroll
+  for (int i = 0; i < V; ++i) {
+    mu = fmaxf(mu, fmaxf(fabsf(v[0][i].x), fmaxf(fabsf(v[0][i].y), fabsf(v[1][i].x))));
+    mb = fmaxf(mb, fmaxf(fabsf(v[1][i].y), fmaxf(fabsf(v[2][i].x), fabsf(v[2][i].y))));
+  }
+  unsigned int bu = __float_as_uint(mu), bb = __float_as_uint(mb);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    bu = max(bu, __shfl_xor_sync(0xffffffffu, bu, o));
+    bb = max(bb, __shfl_xor_sync(0xffffffffu, bb, o));
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(vm, bu);
+    atomicMax(vm + 1, bb);
+  }
+}
 
 // Fused x pass: per physical row (z, y): 3 inverse c2r pairs -> 6 physical fields -> 8 products
 // -> 4 forward r2c pairs -> 8 half-spectrum rows, written back over the same row slots.
@@ -628,7 +731,10 @@ struct XCfg {
 // HDX (hydrodynamics, HDcalcN!): three fields in (ux uy | uz), B = 0 folded at compile time, two
 // inverse and three forward transforms; the products are the first five of the MHD set (the
 // sixth slot written is zero).
-template <class P, int GROUPS, int NTI, int NTF, int MINB, int VPM = 0, bool HDX = false, bool DIRECT = false>
+// PLANE: the rows lie in plane order (kx modes n^2 apart, rows of consecutive y adjacent: rowstride
+// 1, slot stride Kx n^2), read straight into registers (DIRECT).
+template <class P, int GROUPS, int NTI, int NTF, int MINB, int VPM = 0, bool HDX = false, bool DIRECT = false,
+          bool PLANE = false>
 __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     x_fused_kernel(float2* pool, Geom geo, long long rowstride, long long slot, long long istride, BatchRef br,
                    const float2* __restrict__ tw, const float2* __restrict__ twr, unsigned int* vmax, VpRef vp) {
@@ -638,6 +744,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   static_assert(NTI == 1 || NTI == 3, "inverse transforms go one or three at a time");
   static_assert(NTF == 1 || NTF == 2 || NTF == 4, "forward transforms go one, two or four at a time");
   static_assert(NTF == 1 || P::G <= 32, "batched forward transforms need the row inside one warp");
+  static_assert(!PLANE || (DIRECT && P::G <= 32), "plane order is read directly, a row inside one warp");
   static_assert(VPM == 0 || NTF == 1, "the penalty pairs go one at a time");
   static_assert(!HDX || (NTI == 1 && NTF == 1), "the hydrodynamic form goes one transform at a time");
   // forward transform pairs per row; the hydrodynamic form with penalisation fills the three
@@ -647,6 +754,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   constexpr int NINV = HDX ? 2 : 3;             // inverse transforms (field pairs) per row
   constexpr int G = P::G, V = P::V, N = P::N, RPG = XC::RPG, TPG = XC::TPG, TS = XC::TS;
   constexpr int KX = kept_kx_of(N);  // the host checks geo.kx == KX
+  constexpr int XS = PLANE ? N * N : 1;
   extern __shared__ float2 smem[];
   const int kxp = geo.kxp;
   const int grp = threadIdx.x / TPG;
@@ -685,7 +793,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   for (int it = 0; q < ngroups; q += qstep, ++it) {
     const float2* rin;
     if constexpr (DIRECT) {
-      // this row's own slots (slot stride == kxp); every lane loads its inputs before any lane
+      // this row's own slots; every lane loads its inputs before any lane
       // stores an output over them (the stores follow the transforms)
       rin = group_rows(q) + rr * rowstride;
     } else {
@@ -696,11 +804,13 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       sync();
       rin = cur + rr * 6 * kxp;
     }
+    const long long rs = PLANE ? slot : (long long)kxp;  // field stride of the row's inputs
     float2 v[3][V];
 #pragma unroll
     for (int t = 0; t < NINV; ++t) {
-      if (HDX && t == 1) load_herm_pair<P, KX, true>(v[t], rin + (2 * t) * kxp, nullptr, g);
-      else load_herm_pair<P, KX>(v[t], rin + (2 * t) * kxp, rin + (2 * t + 1) * kxp, g);
+      const RowRead<XS> f1{rin + (2 * t) * rs}, f2{rin + (2 * t + 1) * rs};
+      if (HDX && t == 1) load_herm_pair<P, KX, true>(v[t], f1, f2, g);
+      else load_herm_pair<P, KX>(v[t], f1, f2, g);
     }
     if constexpr (NTI == 3) {
       fft_run<P, +1, 3, TS, 1, false>(v, sb, 0, g, tw, sync);
@@ -720,25 +830,8 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       }
     }
     if (vmax) {
-      // max |u_i| and max |B_i| over the physical fields (getCFL! on the last stage's fields);
-      // non-negative floats order like their bit patterns, NaN above +inf
-      float mu = 0.f, mb = 0.f;
-#pragma unroll
-      for (int i = 0; i < V; ++i) {
-        mu = fmaxf(mu, fmaxf(fabsf(v[0][i].x), fmaxf(fabsf(v[0][i].y), fabsf(v[1][i].x))));
-        mb = fmaxf(mb, fmaxf(fabsf(v[1][i].y), fmaxf(fabsf(v[2][i].x), fabsf(v[2][i].y))));
-      }
-      unsigned int bu = __float_as_uint(mu), bb = __float_as_uint(mb);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        bu = max(bu, __shfl_xor_sync(0xffffffffu, bu, o));
-        bb = max(bb, __shfl_xor_sync(0xffffffffu, bb, o));
-      }
-      if ((threadIdx.x & 31) == 0) {
-        const int inst = (int)((ngroups - 1 - q) / GPI);  // the instance of group_rows(q)
-        atomicMax(vmax + 2 * br.list[inst], bu);
-        atomicMax(vmax + 2 * br.list[inst] + 1, bb);
-      }
+      const int inst = (int)((ngroups - 1 - q) / GPI);  // the instance of group_rows(q)
+      x_vmax(v, vmax + 2 * br.list[inst]);
     }
     float2* rowp = group_rows(q) + rr * rowstride;
     // the penalty inputs of this row at the physical points this thread holds: x = lF + LF e for
@@ -763,53 +856,16 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     for (int t0 = 0; t0 < NPAIR; t0 += NTF) {
       float2 w[NTF][V];
 #pragma unroll
-      for (int j = 0; j < NTF; ++j) {
-        const int t = t0 + j;
-#pragma unroll
-        for (int i = 0; i < V; ++i) {
-          const float ux = v[0][i].x, uy = v[0][i].y, uz = v[1][i].x;
-          const float bx = v[1][i].y, by = v[2][i].x, bz = v[2][i].y;
-          if (HDX && VPM > 0 && t >= 2) {
-            if constexpr (HDX && VPM > 0) {
-              constexpr float n3 = (float)N * (float)N * (float)N;
-              const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
-              auto wall = [&](int c) { return VPM == 2 ? n3 * __ldg(wrow + c * vp.cs + x) : 0.f; };
-              // scaled by n^3 to the products' magnitude (n^6 times physical): a pair whose halves
-              // differ by n^3 would lose the small half to the large one's rounding in the split
-              const float c3 = n3 * chi[i];
-              if (t == 2) w[j][i] = make_float2(-uy * uz, c3 * (uz - wall(2)));
-              else w[j][i] = make_float2(c3 * (ux - wall(0)), c3 * (uy - wall(1)));
-            }
-          } else if (t >= 4) {  // penalty pair t - 4: (u x, u y), (u z, B x), (B y, B z) of the field pairs
-            if constexpr (VPM > 0) {
-              float2 f = v[t - 4][i];
-              if constexpr (VPM == 2) {  // the fields are n^3 times physical: so are the walls
-                constexpr float n3 = (float)N * (float)N * (float)N;
-                const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
-                const long long c0 = (long long)(2 * (t - 4)) * vp.cs;
-                f.x = fmaf(-n3, __ldg(wrow + c0 + x), f.x);
-                f.y = fmaf(-n3, __ldg(wrow + c0 + vp.cs + x), f.y);
-              }
-              w[j][i] = make_float2(chi[i] * f.x, chi[i] * f.y);
-            }
-          } else if (t == 0) {
-            const float tzz = bz * bz - uz * uz;
-            w[j][i] = make_float2((bx * bx - ux * ux) - tzz, (by * by - uy * uy) - tzz);
-          } else if (t == 1) {
-            w[j][i] = make_float2(bx * by - ux * uy, bx * bz - ux * uz);
-          } else if (t == 2) {
-            w[j][i] = make_float2(by * bz - uy * uz, ux * by - bx * uy);
-          } else {
-            w[j][i] = make_float2(ux * bz - bx * uz, uy * bz - by * uz);
-          }
-        }
-      }
+      for (int j = 0; j < NTF; ++j) x_pair<P, VPM, HDX>(w[j], t0 + j, v, chi, wrow, vp.cs, g);
       fft_run<PR, -1, NTF, TS, 1>(w, sb, 0, g, twr, sync);
       if constexpr (G <= 32) {
 #pragma unroll
         for (int j = 0; j < NTF; ++j)
-          store_split_shfl<PR, KX>(w[j], g, (threadIdx.x & 31) - g, rowp + (2 * (t0 + j)) * slot,
-                                   rowp + (2 * (t0 + j) + 1) * slot);
+          split_shfl<PR, KX>(w[j], g, (threadIdx.x & 31) - g, [&](int k, float2 a, float2 b) {
+            float2* o = rowp + (2 * (t0 + j)) * slot + k * XS;
+            o[0] = a;
+            o[slot] = b;
+          });
         sync();  // the next transform's first exchange overwrites sb
       } else {
         sync();
@@ -831,7 +887,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
 
 // Plain c2r of row pairs: spectral rows (2q, 2q+1) -> physical rows times scale (1/n^3: the
 // column passes do not normalise).
-template <class P, int ROWS>
+template <class P, int ROWS, bool PLANE = false>
 __global__ void __launch_bounds__(ROWS * P::G) x_c2r_kernel(const float2* src, float* dst, Geom geo, long long srow,
                                                               float scale, const float2* __restrict__ tw) {
   constexpr int G = P::G, V = P::V, N = P::N;
@@ -840,7 +896,8 @@ __global__ void __launch_bounds__(ROWS * P::G) x_c2r_kernel(const float2* src, f
   const int r = threadIdx.x / G, g = threadIdx.x % G;
   const long long q = (long long)blockIdx.x * ROWS + r;
   float2 v[1][V];
-  load_herm_pair<P, kept_kx_of(P::N)>(v[0], src + (2 * q) * srow, src + (2 * q + 1) * srow, g);
+  constexpr int XS = PLANE ? N * N : 1;
+  load_herm_pair<P, kept_kx_of(P::N)>(v[0], RowRead<XS>{src + (2 * q) * srow}, RowRead<XS>{src + (2 * q + 1) * srow}, g);
   fft_run<P, +1, 1, TS, 1, false>(v, smem + r * TS, 0, g, tw, RowSync<G>{1 + r});
   float* da = dst + (2 * q) * N;
   float* db = dst + (2 * q + 1) * N;
@@ -855,7 +912,7 @@ __global__ void __launch_bounds__(ROWS * P::G) x_c2r_kernel(const float2* src, f
 }
 
 // Plain r2c of row pairs: physical rows (2q, 2q+1) -> half-spectrum rows (kx kept modes).
-template <class P, int ROWS>
+template <class P, int ROWS, bool PLANE = false>
 __global__ void __launch_bounds__(ROWS * P::G) x_r2c_kernel(const float* src, float2* dst, Geom geo, long long drow,
                                                               const float2* __restrict__ tw) {
   constexpr int G = P::G, V = P::V, N = P::N;
@@ -885,7 +942,7 @@ __global__ void __launch_bounds__(ROWS * P::G) x_r2c_kernel(const float* src, fl
       if (k < geo.kx || k > N - geo.kx) sb[k] = v[0][d * P::RF + e];
     }
   sync();
-  store_split_pair(sb, N, geo.kx, g, G, dst + (2 * q) * drow, dst + (2 * q + 1) * drow);
+  store_split_pair<PLANE ? N * N : 1>(sb, N, geo.kx, g, G, dst + (2 * q) * drow, dst + (2 * q + 1) * drow);
 }
 
 }  // namespace mhdgb

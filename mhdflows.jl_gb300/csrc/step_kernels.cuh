@@ -20,10 +20,8 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo
   const unsigned int i = 2u * (blockIdx.x * kStageThreads + threadIdx.x);
   if ((int)blockIdx.z >= *br.count) return;
   const int slot = br.list[blockIdx.z];
-  const unsigned int row = i / (unsigned int)geo.kxp;  // a compact field has fewer than 2^32 elements
-  const int x = (int)(i - row * (unsigned int)geo.kxp), jz = (int)(row / (unsigned int)geo.k2);
-  const int jy = (int)(row - (unsigned int)jz * (unsigned int)geo.k2);
-  if (jz >= geo.k2 || x >= geo.kx) return;
+  int x, jy, jz;
+  if (i >= field_elems(geo) || !mode_at(geo, i, x, jy, jz)) return;
   const int t = blockIdx.y;
   const long long so = slot * a.stI + 3 * t * a.fs + i;
   const float2* X = a.X + so;
@@ -49,26 +47,26 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo
   const SlotParams sp = a.sp[slot];
   const RkSlot rs{rs0.sol, rs0.acc, rs0.xn, a.hf * sp.dt, sp.dt, sp.dt / 6.f, a.ca, a.cb};
   // the kx = 0 plane diffuses its Hermitian part, H[f][kz'][ky'] (written before X is updated)
-  const long long hpl = (long long)geo.k2 * geo.k2;
-  const float2* H = a.H + slot * a.hI + 3 * t * hpl + jz * geo.k2 + jy;
+  const long long hrow = geo.planar ? geo.k2p : geo.k2, hpl = hrow * geo.k2;
+  const float2* H = a.H + slot * a.hI + 3 * t * hpl + jz * hrow + jy;
   float2 nx[3][2], ac[3][2];
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     auto half = [&](const float4& v) { return h ? make_float2(v.z, v.w) : make_float2(v.x, v.y); };
-    const int xh = x + h;
+    const int xh = geo.planar ? x : x + h, yh = geo.planar ? jy + h : jy;
     float2 p[5], pen[3], d[3], R[3];
 #pragma unroll
     for (int q = 0; q < 5; ++q) p[q] = half(pl[q]);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       d[c] = half(xv[c]);
-      if (xh == 0) d[c] = H[c * hpl];
+      if (xh == 0) d[c] = H[c * hpl + (geo.planar ? h : 0)];
       if constexpr (GENERAL) pen[c] = half(pn[c]);
     }
     const float kxv = geo.kscale * (float)xh;
-    const float kyv = geo.kscale * (float)signed_of_kept(geo, jy);
+    const float kyv = geo.kscale * (float)signed_of_kept(geo, yh);
     const float kzv = geo.kscale * (float)signed_of_kept(geo, jz);
-    triple_rhs<GENERAL, HD>(a, geo, sp, slot, t, xh, jy, jz, kxv, kyv, kzv, d, p, pen, R);
+    triple_rhs<GENERAL, HD>(a, geo, sp, slot, t, xh, yh, jz, kxv, kyv, kzv, d, p, pen, R);
 #pragma unroll
     for (int c = 0; c < 3; ++c) nx[c][h] = stage_update(OP, rs, half(xv[c]), R[c], half(s4[c]), half(q4[c]), ac[c][h]);
   }
@@ -129,21 +127,20 @@ __global__ void maxabs_into_kernel(const float* __restrict__ a, long long n, uns
 // Layout conversion between the reference's column-major sol[kx, ky, kz, f] (half spectrum,
 // nkr = n/2+1) and the compact retained-band state.
 // ------------------------------------------------------------------------------------------
+// Retained modes of the reference layout -> compact state, walked in the reference's order (kx
+// fastest), so that the reads, which may cross the host link, are contiguous; padding elements
+// of S are never read and keep the zeros of their allocation.
 __global__ void gather_state_kernel(const float2* __restrict__ ref, float2* __restrict__ S, Geom geo, int nf) {
-  const long long total = (long long)nf * geo.k2 * geo.k2 * geo.kxp;
+  const long long total = (long long)nf * geo.k2 * geo.k2 * geo.kx;
   const int nkr = geo.n / 2 + 1;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % geo.kxp);
-    long long r = i / geo.kxp;
+    const int x = (int)(i % geo.kx);
+    long long r = i / geo.kx;
     const int jy = (int)(r % geo.k2); r /= geo.k2;
     const int jz = (int)(r % geo.k2);
     const int f = (int)(r / geo.k2);
-    float2 val = make_float2(0.f, 0.f);
-    if (x < geo.kx) {
-      const int fy = freq_of_kept(geo, jy), fz = freq_of_kept(geo, jz);
-      val = ref[(((long long)f * geo.n + fz) * geo.n + fy) * nkr + x];
-    }
-    S[i] = val;
+    const int fy = freq_of_kept(geo, jy), fz = freq_of_kept(geo, jz);
+    S[f * geo.fs + mode_off(geo, x, jy, jz)] = ref[(((long long)f * geo.n + fz) * geo.n + fy) * nkr + x];
   }
 }
 
@@ -155,7 +152,7 @@ __device__ __forceinline__ float2 ref_value(const float2* __restrict__ S, const 
   const int fz = (int)(r % geo.n);
   const int f = (int)(r / geo.n);
   const int jy = kept_of_freq(geo, fy), jz = kept_of_freq(geo, fz);
-  if (x < geo.kx && jy >= 0 && jz >= 0) return S[(((long long)f * geo.k2 + jz) * geo.k2 + jy) * geo.kxp + x];
+  if (x < geo.kx && jy >= 0 && jz >= 0) return S[f * geo.fs + mode_off(geo, x, jy, jz)];
   return make_float2(0.f, 0.f);
 }
 
@@ -184,7 +181,7 @@ __global__ void scatter_retained_kernel(const float2* __restrict__ S, float2* __
     const int jz = (int)(r % geo.k2);
     const int f = (int)(r / geo.k2);
     const long long row = ((long long)f * geo.n + freq_of_kept(geo, jz)) * geo.n + freq_of_kept(geo, jy);
-    ref[row * nkr + x] = S[(((long long)f * geo.k2 + jz) * geo.k2 + jy) * geo.kxp + x];
+    ref[row * nkr + x] = S[f * geo.fs + mode_off(geo, x, jy, jz)];
   }
 }
 
@@ -220,14 +217,11 @@ __device__ __forceinline__ void block_reduce_diag(double (&acc)[kDiagSlots], dou
 }
 
 __global__ void __launch_bounds__(kDiagThreads) diag_partial_kernel(const float2* __restrict__ S, Geom geo, double* partial) {
-  const long long plane = (long long)geo.k2 * geo.k2 * geo.kxp;  // one field
+  const long long plane = field_elems(geo);
   double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % geo.kxp);
-    if (x >= geo.kx) continue;
-    long long r = i / geo.kxp;
-    const int jy = (int)(r % geo.k2);
-    const int jz = (int)(r / geo.k2);
+    int x, jy, jz;
+    if (!mode_at(geo, i, x, jy, jz)) continue;
     const double w = x == 0 ? 1.0 : 2.0;
     const double kx = (double)geo.kscale * x;
     const double ky = (double)geo.kscale * signed_of_kept(geo, jy);
@@ -237,7 +231,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_partial_kernel(const float2
     bool bad = false;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const float2 u = S[c * plane + i], b = S[(c + 3) * plane + i];
+      const float2 u = S[c * geo.fs + i], b = S[(c + 3) * geo.fs + i];
       bad |= !isfinite(u.x) || !isfinite(u.y) || !isfinite(b.x) || !isfinite(b.y);
       eu += (double)u.x * u.x + (double)u.y * u.y;
       eb += (double)b.x * b.x + (double)b.y * b.y;
@@ -278,14 +272,11 @@ __global__ void __launch_bounds__(kDiagThreads) diag_partial_batch_kernel(const 
   if (inst >= *br.count) return;
   const int slot = br.list[inst];
   const float2* S = pool + slot * stI;
-  const long long plane = (long long)geo.k2 * geo.k2 * geo.kxp;
+  const long long plane = field_elems(geo);
   double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % geo.kxp);
-    if (x >= geo.kx) continue;
-    long long r = i / geo.kxp;
-    const int jy = (int)(r % geo.k2);
-    const int jz = (int)(r / geo.k2);
+    int x, jy, jz;
+    if (!mode_at(geo, i, x, jy, jz)) continue;
     const double w = x == 0 ? 1.0 : 2.0;
     const double kx = (double)geo.kscale * x;
     const double ky = (double)geo.kscale * signed_of_kept(geo, jy);
@@ -295,7 +286,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_partial_batch_kernel(const 
     bool bad = false;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const float2 u = S[c * plane + i], b = S[(c + 3) * plane + i];
+      const float2 u = S[c * geo.fs + i], b = S[(c + 3) * geo.fs + i];
       bad |= !isfinite(u.x) || !isfinite(u.y) || !isfinite(b.x) || !isfinite(b.y);
       eu += (double)u.x * u.x + (double)u.y * u.y;
       eb += (double)b.x * b.x + (double)b.y * b.y;
@@ -356,31 +347,28 @@ __global__ void hist_tick_kernel(int* count) {
 
 // i k.B into a one-field compact buffer (input of the div B inverse transform).
 __global__ void divb_spectrum_kernel(const float2* __restrict__ S, float2* __restrict__ out, Geom geo) {
-  const long long plane = (long long)geo.k2 * geo.k2 * geo.kxp;
+  const long long plane = field_elems(geo);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % geo.kxp);
-    long long r = i / geo.kxp;
-    const int jy = (int)(r % geo.k2);
-    const int jz = (int)(r / geo.k2);
+    int x, jy, jz;
+    const bool in = mode_at(geo, i, x, jy, jz);
     const float kx = geo.kscale * x, ky = geo.kscale * signed_of_kept(geo, jy), kz = geo.kscale * signed_of_kept(geo, jz);
-    const float2 bx = S[3 * plane + i], by = S[4 * plane + i], bz = S[5 * plane + i];
+    const float2 bx = S[3 * geo.fs + i], by = S[4 * geo.fs + i], bz = S[5 * geo.fs + i];
     const float re = kx * bx.x + ky * by.x + kz * bz.x;
     const float im = kx * bx.y + ky * by.y + kz * bz.y;
-    out[i] = x < geo.kx ? make_float2(-im, re) : make_float2(0.f, 0.f);
+    out[i] = in ? make_float2(-im, re) : make_float2(0.f, 0.f);
   }
 }
 
 // DivVCorrection! / DivBCorrection! (src/Solver/VPSolver.jl:60-138): u (mask bit 0) and B (bit 1)
 // of every active slot lose their gradient part, X -= k (k.X) / k^2 with 1/k^2 = 0 at k = 0.
-// grid (ceil(kx / blockDim.x), k2, k2 * cap): one thread per retained mode.
+// grid (ceil(field_elems / blockDim.x), cap): one thread per element of a compact field.
 __global__ void div_correct_kernel(float2* __restrict__ pool, Geom geo, long long fs, long long stI, BatchRef br,
                                    int mask) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= geo.kx) return;
-  const int inst = blockIdx.z / geo.k2;
-  if (inst >= *br.count) return;
-  const int jy = blockIdx.y, jz = blockIdx.z - inst * geo.k2;
-  float2* X = pool + br.list[inst] * stI + ((long long)jz * geo.k2 + jy) * geo.kxp + x;
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int inst = blockIdx.y;
+  int x, jy, jz;
+  if (i >= field_elems(geo) || inst >= *br.count || !mode_at(geo, i, x, jy, jz)) return;
+  float2* X = pool + br.list[inst] * stI + i;
   const float kx = geo.kscale * (float)x;
   const float ky = geo.kscale * (float)signed_of_kept(geo, jy);
   const float kz = geo.kscale * (float)signed_of_kept(geo, jz);

@@ -1,0 +1,68 @@
+"""Plane passes and x-row tiles of the small grids: every kernel variant of every form, at every
+size they are compiled for, against the FP64 oracle's right-hand side (relative L2 <= 1e-5 on the
+retained band, the tolerance of the other right-hand-side tests), and the fused stage update of
+both schemes against the oracle's steps.  The kept counts of these sizes end inside, at and next
+to the transform groups, rows and column rounds of the kernels."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def _problem(pkg, mo, n, form, scheme="RK4", dt=1e-3):
+    g = mo.Grid(n)
+    hd, vp = form.startswith("hd"), form.endswith("vp")
+    s = mo.random_spectrum_state(g, seed=300 + n).astype(np.complex64)
+    if hd:
+        s[3:] = 0
+    prob = pkg.Problem(pkg.GPU(0), nx=n, Lx=2 * math.pi, nu=1e-3, eta=0.0 if hd else 2e-3, dt=dt, stepper=scheme,
+                       B_field=not hd, VP_method=vp)
+    prob.set_sol(s[:prob.nfields].T)
+    pen = None
+    if vp:
+        x, y, z = g.mesh()
+        chi = (0.5 * (1 - np.tanh((np.sqrt(x ** 2 + (y - 0.3) ** 2 + z ** 2) - 1.2) / 0.25))).astype(np.float32)
+        wall = tuple((0.3 * (i + 1) * np.sin(x + i) * np.cos(y - z)).astype(np.float32) for i in range(3))
+        prob.set_vp(chi.T, U0=tuple(a.T for a in wall))
+        pen = dict(chi=chi.astype(np.float64), U0=tuple(a.astype(np.float64) for a in wall))
+    return g, s, prob, pen
+
+
+@pytest.mark.parametrize("form", ["mhd", "hd", "mhdvp", "hdvp"])
+@pytest.mark.parametrize("n", [16, 32, 48, 64, 96, 128])
+def test_every_variant_of_every_form(pkg, mo, n, form):
+    g, s, prob, pen = _problem(pkg, mo, n, form)
+    ref = np.zeros(s.shape, dtype=np.complex128)
+    mo.calcN_fast(ref, s.astype(np.complex128), g, 1e-3, 0.0 if form.startswith("hd") else 2e-3,
+                  vp=None if pen is None else dict(pen, dt=1e-3))
+    mask, nf = g.retained_mask(), prob.nfields
+    with prob:
+        for cls, (selected, names) in pkg.variants(prob).items():
+            for i, name in enumerate(names):
+                try:
+                    pkg.select_variant(prob, cls, i)
+                except pkg.MHDError:
+                    continue  # another form's variant
+                got = prob.rhs_c()
+                err = mo.rel_l2(got, ref[:nf], mask)
+                assert err < TOL, f"{cls} {name}: rel L2 {err:.2e}"
+                assert not got[:, ~mask].any()
+            pkg.select_variant(prob, cls, names.index(selected))
+
+
+@pytest.mark.parametrize("scheme", ["RK4", "LSRK4"])
+@pytest.mark.parametrize("n", [16, 48, 64, 96, 128])
+def test_steps(pkg, mo, n, scheme):
+    g, s, prob, _ = _problem(pkg, mo, n, "mhd", scheme)
+    with prob:
+        pkg.stepforward(prob, 2)
+        got = prob.sol_c()
+    st = mo.Stepper(g, 1e-3, 2e-3, 1e-3, scheme, literal=False)
+    ref = s.astype(np.complex128)
+    for _ in range(2):
+        st.stepforward(ref)
+    assert mo.rel_l2(got, ref, g.retained_mask()) < TOL
