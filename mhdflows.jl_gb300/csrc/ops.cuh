@@ -80,7 +80,9 @@ struct ColVariant {
   size_t tw = 0;
   size_t smem = 0;
   int ctas_inv = 0, ctas_fwd = 0;
+  int pref = 0;  // default of the classes whose bit is set (kDefault*)
 };
+constexpr int kDefaultZinv = 1, kDefaultYinv = 2, kDefaultYfwd = 4, kDefaultZfwd = 8;
 
 // Plane passes of a small grid (plane_kernels.cuh): one plan and block size; the stage kernel in
 // its plain form, with penalty planes or forcing, and the hydrodynamic form.
@@ -352,7 +354,7 @@ class Ops : public OpsBase {
   // column passes (y and z): plan C, TX kx columns per tile, MINB CTAs per SM, NBUF tile buffers
   // TWS: stage twiddles in shared memory (behind the tiles)
   template <class C, int TX, int MINB, int NBUF = 2, bool TWS = false>
-  void add_col() {
+  void add_col(int pref = 0) {
     ColVariant c;
     c.name = "col:" + plan_name<C>() + "/tx" + std::to_string(TX) + "/b" + std::to_string(MINB) +
              (NBUF == 2 ? std::string() : "/q" + std::to_string(NBUF)) + (TWS ? "/ts" : "");
@@ -362,12 +364,13 @@ class Ops : public OpsBase {
     c.tx = TX;
     c.smem = sizeof(float2) * (NBUF * (size_t)N * TX + (TWS ? PlanTw<C>::SIZE : 0));
     c.tw = twiddles<C>();
+    c.pref = pref;
     cv.push_back(c);
   }
 
   // TMA-fed column passes (16 kx columns: 128-byte box rows keep every box destination aligned)
   template <class C, int MINB, int NBUF, bool TWS = false>
-  void add_col_tma() {
+  void add_col_tma(int pref = 0) {
     constexpr int TX = 16;
     ColVariant c;
     c.name = "coltma:" + plan_name<C>() + "/tx" + std::to_string(TX) + "/b" + std::to_string(MINB) + "/q" +
@@ -379,6 +382,7 @@ class Ops : public OpsBase {
     c.smem = sizeof(float2) * NBUF * (size_t)N * TX + NBUF * sizeof(unsigned long long) + 16 +
              (TWS ? sizeof(float2) * PlanTw<C>::SIZE : 0);
     c.tw = twiddles<C>();
+    c.pref = pref;
     cv.push_back(c);
   }
 

@@ -92,13 +92,19 @@ int OpsBase::setup(const Geom& g) {
   if (!cv.empty() && cv[0].inv_tma) return report_error(MHD_ERR_INVALID, "the default column variant must not be TMA-fed");
   if ((rc = set_smem(planar ? (const void*)c2r_plane : (const void*)c2r, row_smem))) return rc;
   if ((rc = set_smem(planar ? (const void*)r2c_plane : (const void*)r2c, row_smem))) return rc;
-  // the default of each class is its first variant that fits on this device
+  // the default of each class is its first variant that fits on this device and names the class as its
+  // own, else the first that fits
   for (int cls = 0; cls < kTunedClasses; ++cls) {
     int i = 0;
     while (i < variant_count(cls) && !variant_ok(cls, i)) ++i;
     if (planar && plane_cls(cls))  // or the first that is meant for this class and capacity
       for (int j = i; j < variant_count(cls); ++j)
         if (variant_ok(cls, j) && (pv[j].pref >> (is_inv(cls) ? 0 : 1) >> (batch ? 2 : 0) & 1)) { i = j; break; }
+    if (!planar && is_col(cls)) {
+      const int bit = cls == KC_ZINV ? kDefaultZinv : cls == KC_YINV ? kDefaultYinv : cls == KC_YFWD ? kDefaultYfwd : kDefaultZfwd;
+      for (int j = i; j < variant_count(cls); ++j)
+        if (variant_ok(cls, j) && (cv[j].pref & bit)) { i = j; break; }
+    }
     if (i == variant_count(cls))
       return report_error(cls == KC_XFUSED && prec ? MHD_ERR_INVALID : MHD_ERR_CUDA,
                           cls == KC_XFUSED && prec ? "no x-row kernel of this precision form for this grid size"
