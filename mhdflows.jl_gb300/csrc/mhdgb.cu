@@ -1370,6 +1370,19 @@ bool is_device_memory(const void* p) {
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Layout conversions of nf fields (step_kernels.cuh): a z-plane of a field per block row, a thread
+// per element (gather, retained scatter) or pair.
+dim3 copy_grid(long long elems, int planes) { return dim3((unsigned)((elems + kCopyThreads - 1) / kCopyThreads), planes); }
+void gather_state(mhd_handle h, const float2* ref, float2* S, int nf, cudaStream_t s) {
+  if (nf > 0) gather_state_kernel<<<copy_grid(((long long)h->g.k2 * h->g.kx + 3) / 4, nf * h->g.k2), kCopyThreads, 0, s>>>(ref, S, h->g);
+}
+void scatter_state(mhd_handle h, const float2* S, float2* ref, int nf, cudaStream_t s) {
+  scatter_state_kernel<<<copy_grid((long long)h->g.n * (h->g.n / 2 + 1) / 2, nf * h->g.n), kCopyThreads, 0, s>>>(S, ref, h->g);
+}
+void scatter_retained(mhd_handle h, const float2* S, float2* ref, int nf, cudaStream_t s) {
+  if (nf > 0) scatter_retained_kernel<<<copy_grid(((long long)h->g.k2 * h->g.kx + 3) / 4, nf * h->g.k2), kCopyThreads, 0, s>>>(S, ref, h->g);
+}
+
 }  // namespace
 
 extern "C" {
@@ -1395,17 +1408,17 @@ int mhd_slot_set_state(mhd_handle h, int slot, const float* sol) {
                                         nf - hf, cudaMemcpyHostToDevice, h->zstream);
     if (e != cudaSuccess) return fail(MHD_ERR_CUDA, std::string("set_state copy: ") + cudaGetErrorString(e));
     MHD_CUDA(cudaEventRecord(h->ev_z, h->zstream));
-    if ((rc = h->launch(KC_OTHER, [&] { gather_state_kernel<<<1216, 256, 0, h->stream>>>(mapped, dst, h->g, hf); }))) return rc;
+    if ((rc = h->launch(KC_OTHER, [&] { gather_state(h, mapped, dst, hf, h->stream); }))) return rc;
     MHD_CUDA(cudaStreamWaitEvent(h->stream, h->ev_z, 0));
     if ((rc = h->launch(KC_OTHER, [&] {
-           gather_state_kernel<<<1216, 256, 0, h->stream>>>(h->ref + hf * fref, dst + hf * h->sz.fs, h->g, nf - hf);
+           gather_state(h, h->ref + hf * fref, dst + hf * h->sz.fs, nf - hf, h->stream);
          })))
       return rc;
   } else {
     // only the retained band crosses the link (29% of the array), into the staging array
     const cudaError_t e = copy_retained(h->ref, sol, h->g, nf, cudaMemcpyHostToDevice, h->stream);
     if (e != cudaSuccess) return fail(MHD_ERR_CUDA, std::string("set_state copy: ") + cudaGetErrorString(e));
-    if ((rc = h->launch(KC_OTHER, [&] { gather_state_kernel<<<1216, 256, 0, h->stream>>>(h->ref, dst, h->g, nf); }))) return rc;
+    if ((rc = h->launch(KC_OTHER, [&] { gather_state(h, h->ref, dst, nf, h->stream); }))) return rc;
   }
   MHD_CUDA(cudaStreamSynchronize(h->stream));
   return MHD_OK;
@@ -1423,7 +1436,7 @@ int mhd_slot_get_state(mhd_handle h, int slot, float* sol) {
   if (out && bytes < (size_t(16) << 20)) {
     // small mapped buffers: the device writes every element
     if ((rc = h->launch(KC_OTHER, [&] {
-           scatter_state_kernel<<<1216, 256, 0, h->stream>>>(src, out, h->g, nf);
+           scatter_state(h, src, out, nf, h->stream);
          })))
       return rc;
   } else if (out) {
@@ -1440,14 +1453,14 @@ int mhd_slot_get_state(mhd_handle h, int slot, float* sol) {
     if (zp != ZeroPath::Host)
       MHD_CUDA(zero_alias_blocks(host, h->g, nf, h->zeros, h->zbytes, h->zstream, zp == ZeroPath::CopyEngine));
     if ((rc = h->launch(KC_OTHER, [&] {
-           scatter_retained_kernel<<<1216, 256, 0, h->stream>>>(src + hf * h->sz.fs, h->ref + hf * fref, h->g, nf - hf);
+           scatter_retained(h, src + hf * h->sz.fs, h->ref + hf * fref, nf - hf, h->stream);
          })))
       return rc;
     MHD_CUDA(cudaEventRecord(h->ev_z, h->stream));
     MHD_CUDA(cudaStreamWaitEvent(h->zstream, h->ev_z, 0));
     MHD_CUDA(copy_retained(host + hf * fref, h->ref + hf * fref, h->g, nf - hf, cudaMemcpyDeviceToHost, h->zstream));
     if ((rc = h->launch(KC_OTHER, [&] {
-           scatter_retained_kernel<<<1216, 256, 0, h->stream>>>(src, out, h->g, hf);
+           scatter_retained(h, src, out, hf, h->stream);
          })))
       return rc;
     zero_alias_host(host, h->g, nf, zp == ZeroPath::Host, zp != ZeroPath::CopyEngine);
@@ -1456,7 +1469,7 @@ int mhd_slot_get_state(mhd_handle h, int slot, float* sol) {
     // the full array is assembled in the staging buffer at HBM speed, zeros included, and comes
     // back in one contiguous copy
     if ((rc = h->launch(KC_OTHER, [&] {
-           scatter_state_kernel<<<1216, 256, 0, h->stream>>>(src, h->ref, h->g, nf);
+           scatter_state(h, src, h->ref, nf, h->stream);
          })))
       return rc;
     MHD_CUDA(cudaMemcpyAsync(sol, h->ref, bytes, cudaMemcpyDeviceToHost, h->stream));
@@ -1484,8 +1497,8 @@ static int state_device(mhd_handle h, int slot, float* sol_dev, void* stream, bo
   }
   float2* st = h->sol + slot * h->sz.state;
   float2* ref = reinterpret_cast<float2*>(sol_dev);
-  if (to_state) gather_state_kernel<<<1216, 256, 0, s>>>(ref, st, h->g, h->nfields());
-  else scatter_state_kernel<<<1216, 256, 0, s>>>(st, ref, h->g, h->nfields());
+  if (to_state) gather_state(h, ref, st, h->nfields(), s);
+  else scatter_state(h, st, ref, h->nfields(), s);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MHD_ERR_CUDA, std::string(to_state ? "gather" : "scatter") + " launch: " + cudaGetErrorString(e));
   if (s != h->stream) {
@@ -1867,7 +1880,7 @@ int mhd_compute_rhs(mhd_handle h, float* rhs_out) {
   if (rc) return rc;
   if (!rhs_out) return fail(MHD_ERR_INVALID, "null output");
   if ((rc = h->rhs(h->sol, h->acc, OP_RHS, 0.f, 0.f, 0.f, h->slot_ref(0), 7))) return rc;
-  if ((rc = h->launch(KC_OTHER, [&] { scatter_state_kernel<<<1216, 256, 0, h->stream>>>(h->acc, h->ref, h->g, h->nfields()); }))) return rc;
+  if ((rc = h->launch(KC_OTHER, [&] { scatter_state(h, h->acc, h->ref, h->nfields(), h->stream); }))) return rc;
   MHD_CUDA(cudaMemcpyAsync(rhs_out, h->ref, h->ref_elems() * sizeof(float2), cudaMemcpyDeviceToHost, h->stream));
   MHD_CUDA(cudaStreamSynchronize(h->stream));
   return MHD_OK;

@@ -127,61 +127,65 @@ __global__ void maxabs_into_kernel(const float* __restrict__ a, long long n, uns
 // Layout conversion between the reference's column-major sol[kx, ky, kz, f] (half spectrum,
 // nkr = n/2+1) and the compact retained-band state.
 // ------------------------------------------------------------------------------------------
-// Retained modes of the reference layout -> compact state, walked in the reference's order (kx
-// fastest), so that the reads, which may cross the host link, are contiguous; padding elements
-// of S are never read and keep the zeros of their allocation.
-__global__ void gather_state_kernel(const float2* __restrict__ ref, float2* __restrict__ S, Geom geo, int nf) {
-  const long long total = (long long)nf * geo.k2 * geo.k2 * geo.kx;
-  const int nkr = geo.n / 2 + 1;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % geo.kx);
-    long long r = i / geo.kx;
-    const int jy = (int)(r % geo.k2); r /= geo.k2;
-    const int jz = (int)(r % geo.k2);
-    const int f = (int)(r / geo.k2);
-    const int fy = freq_of_kept(geo, jy), fz = freq_of_kept(geo, jz);
-    S[f * geo.fs + mode_off(geo, x, jy, jz)] = ref[(((long long)f * geo.n + fz) * geo.n + fy) * nkr + x];
+// These kernels take one z-plane of one field per blockIdx.y, so that an element's row needs one
+// 32-bit division and no others, and four elements per thread where the accesses are 8 bytes.  With the
+// 64-bit divisions of a flat index by four run-time sizes they ran at a third of HBM's rate: push and
+// pull of prob.sol 80 + 206 us at 256^3 and 579 + 1570 us at 512^3, now 55 + 100 and 373 + 754 us.
+constexpr int kCopyThreads = 256;
+
+// Retained modes of the reference layout -> compact state, in the reference's order (kx fastest), so
+// that the reads, which may cross the host link, are contiguous; padding elements of S are never
+// read and keep the zeros of their allocation.  blockIdx.y = f k2 + kz'.
+__global__ void __launch_bounds__(kCopyThreads) gather_state_kernel(const float2* __restrict__ ref, float2* __restrict__ S,
+                                                                    Geom geo) {
+  const unsigned int kx = geo.kx, total = (unsigned int)geo.k2 * kx;
+  const int nkr = geo.n / 2 + 1, f = blockIdx.y / geo.k2, jz = blockIdx.y - f * geo.k2;
+  const float2* src = ref + ((long long)f * geo.n + freq_of_kept(geo, jz)) * geo.n * nkr;
+  float2* dst = S + f * geo.fs;
+#pragma unroll 4
+  for (unsigned int i = blockIdx.x * kCopyThreads + threadIdx.x; i < total; i += gridDim.x * kCopyThreads) {
+    const int jy = (int)(i / kx), x = (int)(i - (unsigned int)jy * kx);
+    dst[mode_off(geo, x, jy, jz)] = src[freq_of_kept(geo, jy) * nkr + x];
   }
 }
 
-// One element of the reference layout from the compact state (zero in the alias band).
-__device__ __forceinline__ float2 ref_value(const float2* __restrict__ S, const Geom& geo, long long i, int nkr) {
-  const int x = (int)(i % nkr);
-  long long r = i / nkr;
-  const int fy = (int)(r % geo.n); r /= geo.n;
-  const int fz = (int)(r % geo.n);
-  const int f = (int)(r / geo.n);
-  const int jy = kept_of_freq(geo, fy), jz = kept_of_freq(geo, fz);
-  if (x < geo.kx && jy >= 0 && jz >= 0) return S[f * geo.fs + mode_off(geo, x, jy, jz)];
-  return make_float2(0.f, 0.f);
-}
-
-// Compact state -> reference layout, two elements (one 16-byte store) per thread and step: the
-// element count nf n^2 nkr is even and ref is 16-byte aligned, so every pair is aligned.  The
-// output may be mapped host memory, where wide stores use the host link better.
-__global__ void scatter_state_kernel(const float2* __restrict__ S, float2* __restrict__ ref, Geom geo, int nf) {
-  const int nkr = geo.n / 2 + 1;
-  const long long pairs = (long long)nf * geo.n * geo.n * nkr / 2;
-  float4* out = reinterpret_cast<float4*>(ref);
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < pairs; p += (long long)gridDim.x * blockDim.x) {
-    const float2 a = ref_value(S, geo, 2 * p, nkr), b = ref_value(S, geo, 2 * p + 1, nkr);
-    out[p] = make_float4(a.x, a.y, b.x, b.y);
+// Compact state -> reference layout, two elements (one 16-byte store) per thread and step: a plane
+// has n nkr elements, an even number, and ref is 16-byte aligned, so every pair is aligned.  The
+// output may be mapped host memory, where wide stores use the host link better.  blockIdx.y =
+// f n + the plane's frequency index.
+__global__ void __launch_bounds__(kCopyThreads) scatter_state_kernel(const float2* __restrict__ S, float2* __restrict__ ref,
+                                                                     Geom geo) {
+  const unsigned int nkr = geo.n / 2 + 1, pairs = (unsigned int)geo.n * nkr / 2;
+  const int f = blockIdx.y / geo.n, jz = kept_of_freq(geo, blockIdx.y - f * geo.n);
+  const float2* src = S + f * geo.fs;
+  float4* out = reinterpret_cast<float4*>(ref) + (long long)blockIdx.y * pairs;
+  for (unsigned int p = blockIdx.x * kCopyThreads + threadIdx.x; p < pairs; p += gridDim.x * kCopyThreads) {
+    float2 v[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if (jz >= 0) {
+      unsigned int fy = 2 * p / nkr, x = 2 * p - fy * nkr;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int jy = kept_of_freq(geo, fy);
+        if ((int)x < geo.kx && jy >= 0) v[h] = src[mode_off(geo, x, jy, jz)];
+        if (++x == nkr) { x = 0; ++fy; }
+      }
+    }
+    out[p] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
   }
 }
 
 // Compact state -> the retained elements of the reference layout (kx < Kx, ky and kz kept),
-// 8-byte stores; every other element is zero and the caller fills it.
-__global__ void scatter_retained_kernel(const float2* __restrict__ S, float2* __restrict__ ref, Geom geo, int nf) {
-  const int nkr = geo.n / 2 + 1;
-  const long long total = (long long)nf * geo.k2 * geo.k2 * geo.kx;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < total; p += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(p % geo.kx);
-    long long r = p / geo.kx;
-    const int jy = (int)(r % geo.k2); r /= geo.k2;
-    const int jz = (int)(r % geo.k2);
-    const int f = (int)(r / geo.k2);
-    const long long row = ((long long)f * geo.n + freq_of_kept(geo, jz)) * geo.n + freq_of_kept(geo, jy);
-    ref[row * nkr + x] = S[f * geo.fs + mode_off(geo, x, jy, jz)];
+// 8-byte stores; every other element is zero and the caller fills it.  blockIdx.y = f k2 + kz'.
+__global__ void __launch_bounds__(kCopyThreads) scatter_retained_kernel(const float2* __restrict__ S, float2* __restrict__ ref,
+                                                                        Geom geo) {
+  const unsigned int kx = geo.kx, total = (unsigned int)geo.k2 * kx;
+  const int nkr = geo.n / 2 + 1, f = blockIdx.y / geo.k2, jz = blockIdx.y - f * geo.k2;
+  float2* dst = ref + ((long long)f * geo.n + freq_of_kept(geo, jz)) * geo.n * nkr;
+  const float2* src = S + f * geo.fs;
+#pragma unroll 4
+  for (unsigned int i = blockIdx.x * kCopyThreads + threadIdx.x; i < total; i += gridDim.x * kCopyThreads) {
+    const int jy = (int)(i / kx), x = (int)(i - (unsigned int)jy * kx);
+    dst[freq_of_kept(geo, jy) * nkr + x] = src[mode_off(geo, x, jy, jz)];
   }
 }
 
