@@ -434,8 +434,8 @@ struct mhd_problem {
   }
 
   // device work lists: dlist[0..cap) active, dlist[cap..2cap) identity, dlist[2cap] active count, dlist[2cap+1] = 1
-  BatchRef active_ref() const { return BatchRef{dlist, dlist + 2 * cap}; }
-  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 2 * cap + 1}; }
+  BatchRef active_ref() const { return BatchRef{dlist, dlist + 2 * cap, cap == 1}; }
+  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 2 * cap + 1, cap == 1}; }
 
   int sync_lists() {
     if (!list_dirty) return MHD_OK;

@@ -96,6 +96,8 @@ struct RowSync {
 struct BatchRef {
   const int* list;   // active slots
   const int* count;  // number of active slots
+  int single;        // capacity 1: the slot is 0 and needs no load in front of the first data address
+  __device__ __forceinline__ int slot(int inst) const { return single ? 0 : list[inst]; }
 };
 
 // Volume-penalisation inputs of the x rows (src/Solver/VPSolver.jl): per slot the mask chi
@@ -146,7 +148,7 @@ __device__ __forceinline__ void herm_kx0_items(const float2* __restrict__ Xpool,
     const int c = (int)(r / pl);
     const long long p = r - c * pl;
     const int jz = (int)(p / geo.k2), jy = (int)(p - (long long)jz * geo.k2);
-    const int slot = br.list[inst];
+    const int slot = br.slot(inst);
     const float2* X = Xpool + slot * stI + c * fs;
     const int py = kept_of_signed(geo, -signed_of_kept(geo, jy));
     const int pz = kept_of_signed(geo, -signed_of_kept(geo, jz));
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
   auto tile_src = [&](const Cur& c) {
     if (c.inst != src_inst) {
       src_inst = c.inst;
-      src_off = br.list[c.inst] * a.sI;
+      src_off = br.slot(c.inst) * a.sI;
     }
     return a.src + src_off + c.f * a.sF + (long long)c.o * a.sO;
   };
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
     if (kxg < geo.kx) {
       if (inst != dst_inst) {
         dst_inst = inst;
-        dst_off = br.list[inst] * a.dI;
+        dst_off = br.slot(inst) * a.dI;
       }
       float2* dst = a.dst + dst_off + f * a.dF + (long long)o * a.dO + kxg;
 #pragma unroll
@@ -449,7 +451,7 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
       int cc[5] = {c.tx * TX, 0, 0, 0, 0};
       cc[tc.odim] = c.o;
       cc[tc.fdim] = c.f;
-      cc[tc.idim] = br.list[c.inst];
+      cc[tc.idim] = br.slot(c.inst);
       if (PIN) {
         cc[tc.rowdim] = 0;
         tma_load5(smem_u32(buf), &map, cc[0], cc[1], cc[2], cc[3], cc[4], bar);
@@ -507,7 +509,7 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
     if (kxg < geo.kx) {
       if (inst != dst_inst) {  // list lookup only when the instance changes
         dst_inst = inst;
-        dst_off = br.list[inst] * a.dI;
+        dst_off = br.slot(inst) * a.dI;
       }
       float2* dst = a.dst + dst_off + f * a.dF + (long long)o * a.dO + kxg;
 #pragma unroll
@@ -773,7 +775,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   auto group_rows = [&](long long q) {
     q = ngroups - 1 - q;
     const int inst = (int)(q / GPI);
-    return pool + br.list[inst] * istride + (q - (long long)inst * GPI) * RPG * rowstride;
+    return pool + br.slot(inst) * istride + (q - (long long)inst * GPI) * RPG * rowstride;
   };
 
   // rows q*RPG .. q*RPG+RPG-1 -> dst (each row's six fields contiguous)
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     }
     if (vmax) {
       const int inst = (int)((ngroups - 1 - q) / GPI);  // the instance of group_rows(q)
-      x_vmax(v, vmax + 2 * br.list[inst]);
+      x_vmax(v, vmax + 2 * br.slot(inst));
     }
     float2* rowp = group_rows(q) + rr * rowstride;
     // the penalty inputs of this row at the physical points this thread holds: x = lF + LF e for
@@ -841,7 +843,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     if constexpr (VPM > 0) {
       const long long qr = ngroups - 1 - q;  // the group group_rows(q) addresses
       const int inst = (int)(qr / GPI);
-      const long long s = br.list[inst];
+      const long long s = br.slot(inst);
       const long long r = (qr - (long long)inst * GPI) * RPG + rr;  // z n + y
       const float* crow = vp.chi + s * vp.cs + r * N;
       if constexpr (VPM == 2) wrow = vp.wall + 6 * s * vp.cs + r * N;

@@ -152,26 +152,33 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_forward_kernel(PlaneArgs 
   using P = typename C::P;
   constexpr int N = C::N, G = C::G, S = C::S;
   extern __shared__ __align__(16) float2 W[];
-  if ((int)blockIdx.z >= *br.count) return;
-  const int slot = br.list[blockIdx.z];
+  const int active = *br.count, slot = br.slot(blockIdx.z);
   const int x = blockIdx.x, f = blockIdx.y;
   const float2* s = a.src + slot * a.sI + ((long long)f * C::KX + x) * (N * N);
   const int lane = threadIdx.x & 31, g = lane % G;
-  for (int r0 = (threadIdx.x >> 5) * C::RPW; r0 < N; r0 += C::RB) {
-    const int row = r0 + lane / G;
-    float2 v[1][P::V];
+  float2 u[P::V];
+  auto load = [&](int row) {
 #pragma unroll
     for (int d = 0; d < P::DI; ++d)
 #pragma unroll
-      for (int n0 = 0; n0 < P::R0; ++n0) v[0][d * P::R0 + n0] = s[row * N + g + G * d + P::LI * n0];
-    row_fft<C, -1, true>(v[0], W + row * S, lane / G, g, tw);
+      for (int n0 = 0; n0 < P::R0; ++n0) u[d * P::R0 + n0] = s[row * N + g + G * d + P::LI * n0];
+  };
+  // one round: the loads come before the test of the instance and do not wait for its count
+  constexpr bool ONE = C::RB >= N;
+  int r0 = (threadIdx.x >> 5) * C::RPW;
+  if (ONE && r0 < N) load(r0 + lane / G);
+  if ((int)blockIdx.z >= active) return;
+  for (; r0 < N; r0 += C::RB) {
+    const int row = r0 + lane / G;
+    if (!ONE) load(row);
+    row_fft<C, -1, true>(u, W + row * S, lane / G, g, tw);
 #pragma unroll
     for (int d = 0; d < P::DF; ++d)
 #pragma unroll
       for (int e = 0; e < P::RF; ++e) {
         if (plane_alias<C>(G * d + P::LF * e)) continue;
         const int j = plane_kept_at<C>(G * d + P::LF * e, g);
-        if (plane_keeps<C>(G * d + P::LF * e, g)) W[row * S + j] = v[0][d * P::RF + e];
+        if (plane_keeps<C>(G * d + P::LF * e, g)) W[row * S + j] = u[d * P::RF + e];
       }
   }
   __syncthreads();
@@ -263,14 +270,14 @@ __device__ __forceinline__ void plane_inverse(float2* W, float2* out, const floa
 template <class C>
 __global__ void __launch_bounds__(C::T, C::MINB) plane_inverse_kernel(PlaneArgs a, BatchRef br, const float2* __restrict__ tw) {
   extern __shared__ __align__(16) float2 W[];
-  if ((int)blockIdx.z >= *br.count) return;
-  const int slot = br.list[blockIdx.z];
+  const int active = *br.count, slot = br.slot(blockIdx.z);
   const int x = blockIdx.x, f = blockIdx.y;
   const float2* X = a.src + slot * a.sI + f * a.dF + (long long)x * (C::K2 * C::K2P);
   for (int m = threadIdx.x; m < C::K2 * C::K2 / 2; m += C::T) {
     const int jz = m / (C::K2 / 2), jy = 2 * (m % (C::K2 / 2));
     *reinterpret_cast<float4*>(W + plane_freq<C>(jz) * C::S + jy) = *reinterpret_cast<const float4*>(X + jz * C::K2P + jy);
   }
+  if ((int)blockIdx.z >= active) return;
   __syncthreads();
   plane_inverse<C>(W, a.dst + slot * a.dI + ((long long)f * C::KX + x) * (C::N * C::N), tw);
 }
@@ -293,8 +300,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_stage_kernel(RkArgs a, Pl
   constexpr int N = C::N, S = C::S, K2 = C::K2, K2P = C::K2P, T = C::T;
   constexpr int PAIRS = K2 * K2 / 2, NP = (PAIRS + T - 1) / T;
   extern __shared__ __align__(16) float2 W[];
-  if ((int)blockIdx.z >= *br.count) return;
-  const int slot = br.list[blockIdx.z];
+  const int active = *br.count, slot = br.slot(blockIdx.z);
   const int x = blockIdx.x, f = blockIdx.y, t = f / 3, op = a.op;
   const long long so = slot * a.stI + f * a.fs + (long long)x * (K2 * K2P);
   const float2* X = a.X + so;
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_stage_kernel(RkArgs a, Pl
     if (m < PAIRS) xv[i] = *reinterpret_cast<const float4*>(X + jz * K2P + jy);
     xd[i] = xv[i];
   }
+  if ((int)blockIdx.z >= active) return;  // after the first loads, which do not wait for the count
   if (x == 0) {  // X(-k) = 0 when -k lies in the alias band
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
@@ -447,7 +454,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     const unsigned int bar = smem_u32(&bars[b]);
     const int inst = t / PER, r = t - inst * PER;
-    const int y0 = r % (N / C::ROWS) * C::ROWS, z = r / (N / C::ROWS), slot = br.list[inst];
+    const int y0 = r % (N / C::ROWS) * C::ROWS, z = r / (N / C::ROWS), slot = br.slot(inst);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((unsigned int)(C::NIN * KX * 128)) : "memory");
 #pragma unroll
@@ -492,7 +499,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
       }
     }
     const int inst = t / PER, r = t - inst * PER;
-    const int y0 = r % (N / C::ROWS) * C::ROWS, z = r / (N / C::ROWS), slot = br.list[inst];
+    const int y0 = r % (N / C::ROWS) * C::ROWS, z = r / (N / C::ROWS), slot = br.slot(inst);
     if (vmax) x_vmax(v, vmax + 2 * slot);
     float chi[VPM ? V : 1];
     const float* wrow = nullptr;

@@ -18,8 +18,7 @@ constexpr int kStageThreads = 128;
 template <int OP, bool GENERAL, bool HD>
 __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo, BatchRef br) {
   const unsigned int i = 2u * (blockIdx.x * kStageThreads + threadIdx.x);
-  if ((int)blockIdx.z >= *br.count) return;
-  const int slot = br.list[blockIdx.z];
+  const int active = *br.count, slot = br.slot(blockIdx.z);
   int x, jy, jz;
   if (i >= field_elems(geo) || !mode_at(geo, i, x, jy, jz)) return;
   const int t = blockIdx.y;
@@ -44,6 +43,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo
       pn[c] = a.vpen ? __ldcs(reinterpret_cast<const float4*>(prod + pp * a.fs)) : zero4;
     }
   }
+  if ((int)blockIdx.z >= active) return;  // after the loads, which do not wait for the count
   const SlotParams sp = a.sp[slot];
   const RkSlot rs{rs0.sol, rs0.acc, rs0.xn, a.hf * sp.dt, sp.dt, sp.dt / 6.f, a.ca, a.cb};
   // the kx = 0 plane diffuses its Hermitian part, H[f][kz'][ky'] (written before X is updated)
@@ -92,7 +92,7 @@ __global__ void cfl_update_kernel(BatchRef br, SlotParams* sp, unsigned int* vma
                                   float vscale, int advance) {
   const int n = *br.count;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int s = br.list[i];
+    const int s = br.slot(i);
     SlotParams p = sp[s];
     if (advance) t[s] += (double)p.dt;
     const float vm = vscale * fmaxf(__uint_as_float(vmax[2 * s]), __uint_as_float(vmax[2 * s + 1]));
@@ -110,7 +110,7 @@ __global__ void cfl_update_kernel(BatchRef br, SlotParams* sp, unsigned int* vma
 // one step of every active slot taken: advance the per-slot step counters (random forcing)
 __global__ void step_tick_kernel(BatchRef br, long long* steps) {
   const int n = *br.count;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) steps[br.list[i]] += 1;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) steps[br.slot(i)] += 1;
 }
 
 // max |field| of one physical field into vmax[which] (initial fields before the first CFL step).
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_partial_batch_kernel(const 
                                                                           Geom geo, BatchRef br, double* partial) {
   const int inst = blockIdx.y;
   if (inst >= *br.count) return;
-  const int slot = br.list[inst];
+  const int slot = br.slot(inst);
   const float2* S = pool + slot * stI;
   const long long plane = field_elems(geo);
   double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_record_kernel(const double*
                                                                    const double* dtime, double scale) {
   const int inst = blockIdx.x;
   if (inst >= *br.count) return;
-  const int slot = br.list[inst];
+  const int slot = br.slot(inst);
   double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
   const double* p = partial + (long long)slot * nblocks * kDiagSlots;
   for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
@@ -372,7 +372,7 @@ __global__ void div_correct_kernel(float2* __restrict__ pool, Geom geo, long lon
   const int inst = blockIdx.y;
   int x, jy, jz;
   if (i >= field_elems(geo) || inst >= *br.count || !mode_at(geo, i, x, jy, jz)) return;
-  float2* X = pool + br.list[inst] * stI + i;
+  float2* X = pool + br.slot(inst) * stI + i;
   const float kx = geo.kscale * (float)x;
   const float ky = geo.kscale * (float)signed_of_kept(geo, jy);
   const float kz = geo.kscale * (float)signed_of_kept(geo, jz);

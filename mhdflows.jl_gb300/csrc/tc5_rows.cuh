@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(128, 2)
   auto tile_rows = [&](long long q) {  // first row of tile q (taken from the last one down)
     q = ntiles - 1 - q;
     const int inst = (int)(q / GPI);
-    return pool + br.list[inst] * istride + (q - (long long)inst * GPI) * R * rowstride;
+    return pool + br.slot(inst) * istride + (q - (long long)inst * GPI) * R * rowstride;
   };
   auto prefetch = [&](long long q, float2* dst) {
     const float2* src = tile_rows(q);
@@ -374,8 +374,8 @@ __global__ void __launch_bounds__(128, 2)
           }
           if (lane == 0) {
             const int inst = (int)((ntiles - 1 - q) / GPI);
-            atomicMax(vmax + 2 * br.list[inst], bu);
-            atomicMax(vmax + 2 * br.list[inst] + 1, bb);
+            atomicMax(vmax + 2 * br.slot(inst), bu);
+            atomicMax(vmax + 2 * br.slot(inst) + 1, bb);
           }
         }
 #pragma unroll

@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(GROUPS * 32, MINB)
   const int chunks_row = 3 * kxp;
   auto row_ptr = [&](long long q) {
     const int inst = (int)(q / GPI);
-    return pool + br.list[inst] * istride + (q - (long long)inst * GPI) * rowstride;
+    return pool + br.slot(inst) * istride + (q - (long long)inst * GPI) * rowstride;
   };
   auto prefetch = [&](long long q, float2* dst) {
     const float2* src = row_ptr(q);
@@ -574,8 +574,8 @@ __global__ void __launch_bounds__(GROUPS * 32, MINB)
       }
       if (lane == 0) {
         const int inst = (int)(q / GPI);
-        atomicMax(vmax + 2 * br.list[inst], bu);
-        atomicMax(vmax + 2 * br.list[inst] + 1, bb);
+        atomicMax(vmax + 2 * br.slot(inst), bu);
+        atomicMax(vmax + 2 * br.slot(inst) + 1, bb);
       }
     }
     // every product is bounded by 4 max(|u|, |B|)^2
