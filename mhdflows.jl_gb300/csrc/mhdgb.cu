@@ -332,7 +332,7 @@ struct mhd_problem {
   // TMA sources of the column passes (used when a TMA-fed variant is selected) and the device
   // word a timed-out tile wait is recorded in
   TmaPass tm_plane;  // plane order: the R planes
-  TmaPass tm_zinv_sol, tm_zinv_xs, tm_yinv, tm_yfwd, tm_zfwd;
+  TmaPass tm_zinv_sol, tm_zinv_xs, tm_yinv, tm_yfwd, tm_zfwd, tm_prod;
   int* derr = nullptr;
   bool cfl = false;
   double cfl_coef = 0.3;
@@ -494,22 +494,22 @@ struct mhd_problem {
   // compact fields (src + slot*sI, nf fields at stride FS) -> colbuf slots 0..nf-1
   int z_inverse(const float2* src, long long sI, int nf, BatchRef br) {
     ColArgs a{src, colbuf, FS(), (long long)g.kxp, (long long)g.k2 * g.kxp, (long long)g.kxp, SLK(), AZ(), sI, sz.colbuf};
-    // the maps cover all six fields of a pool: only the right-hand side's call can use them
-    const TmaPass* tp = (nf == 6 && sI == ST()) ? (src == sol ? &tm_zinv_sol : src == xs ? &tm_zinv_xs : nullptr) : nullptr;
-    return launch(KC_ZINV, [&] { ops->col(KC_ZINV, a, g, g.k2, nf, br, cap, stream, tp); });
+    // the maps cover the fields of a pool from its first on
+    const TmaPass* tp = sI == ST() ? (src == sol ? &tm_zinv_sol : src == xs ? &tm_zinv_xs : nullptr) : nullptr;
+    return launch(KC_ZINV, [&] { ops->col(KC_ZINV, a, g, g.k2, nf, br, cap, stream, tp, &tm_zfwd); });
   }
   int y_inverse(int nf, BatchRef br) {
     ColArgs a{colbuf, rowbuf, (long long)g.kxp, AZ(), SLK(), (long long)g.kxp, BZ(), SLK(), sz.colbuf, sz.rowbuf};
-    return launch(KC_YINV, [&] { ops->col(KC_YINV, a, g, g.n, nf, br, cap, stream, &tm_yinv); });
+    return launch(KC_YINV, [&] { ops->col(KC_YINV, a, g, g.n, nf, br, cap, stream, &tm_yinv, &tm_yfwd); });
   }
   int x_fused(BatchRef br, unsigned int* vmax) {
     // the six field rows of a physical row are contiguous (slot stride == kxp)
     const VpRef vp{vchi, vwall, sz.phys};
-    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, row_stride(), row_slot(), sz.rowbuf, br, cap, vmax, vp, stream, &tm_plane); });
+    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, row_stride(), row_slot(), sz.rowbuf, br, cap, vmax, vp, derr, stream, &tm_plane); });
   }
   int y_forward(int nf, BatchRef br) {
     ColArgs a{rowbuf, colbuf, (long long)g.kxp, BZ(), SLK(), (long long)g.kxp, AZ(), SLK(), sz.rowbuf, sz.colbuf};
-    return launch(KC_YFWD, [&] { ops->col(KC_YFWD, a, g, g.n, nf, br, cap, stream, &tm_yfwd); });
+    return launch(KC_YFWD, [&] { ops->col(KC_YFWD, a, g, g.n, nf, br, cap, stream, &tm_yfwd, &tm_yinv); });
   }
   // colbuf slots -> compact planes (nf fields/products) at dst + slot*dI, pruned output
   // hx: the stage state whose kx = 0 Hermitian part the pass also writes into aux (the
@@ -521,7 +521,9 @@ struct mhd_problem {
     a.hfs = FS();
     a.hsI = ST();
     a.hoI = FS();
-    return launch(KC_ZFWD, [&] { ops->col(KC_ZFWD, a, g, g.k2, nf, br, cap, stream, &tm_zfwd); });
+    // the map of the destination covers the product planes in rowbuf only
+    const TmaPass* to = dst == rowbuf && dI == sz.rowbuf ? &tm_prod : nullptr;
+    return launch(KC_ZFWD, [&] { ops->col(KC_ZFWD, a, g, g.k2, nf, br, cap, stream, &tm_zfwd, to); });
   }
   // ---- plane order (small grids): planes R[slot][kx][z][y] in rowbuf, products in colbuf
   // compact fields (src + slot*sI, nf fields at stride FS) -> R planes 0..nf-1
@@ -887,6 +889,10 @@ struct mhd_problem {
     set(tm_yinv, colbuf, dc, sc, by_in, TmaCoords{2, 3, 1, 4, (int)kp});      // rows ky', outer z
     set(tm_yfwd, rowbuf, dr, sr, by_out, TmaCoords{2, 3, 1, 4, (int)rb});     // rows y, outer z
     set(tm_zfwd, colbuf, dc, sc, bz_out, TmaCoords{3, 2, 1, 4, (int)rb});     // rows z, outer ky'
+    // compact product planes in rowbuf [slot][p][kz'][ky'][kx]: rows kz', outer ky'
+    const cuuint64_t dp[5] = {kxp, k2, k2, S, C};
+    const cuuint64_t sp[4] = {kxp * E, k2 * kxp * E, (cuuint64_t)sz.fs * E, (cuuint64_t)sz.rowbuf * E};
+    set(tm_prod, rowbuf, dp, sp, bz, TmaCoords{2, 1, 3, 4, (int)kp});
   }
   // a TMA tile wait that timed out on the device (checked where the library synchronises)
   int check_device_error() {
@@ -971,7 +977,6 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   h->ops.reset(make_ops(params->n));
   if (!h->ops) return fail(MHD_ERR_INVALID, "no plan for n");
   h->ops->prec = params->precision;
-  h->ops->vp_capable = params->vp != 0;
   h->ops->hd = h->hd_form() ? 1 : 0;
   h->ops->planar = !h->ops->pv.empty() && params->precision == MHD_PREC_FP32;
   h->g.planar = h->ops->planar ? 1 : 0;

@@ -13,6 +13,7 @@
 #include <string>
 #include <vector>
 
+#include "col_pair.cuh"
 #include "passes.cuh"
 #include "plane_kernels.cuh"
 #include "tc5_rows.cuh"
@@ -28,8 +29,9 @@ constexpr int kTunedClasses = 5;  // z_inverse .. z_forward
 int report_error(int code, const std::string& msg);
 
 using XFn = void (*)(float2*, Geom, long long, long long, long long, BatchRef, const float2*, const float2*,
-                     unsigned int*, VpRef);
+                     unsigned int*, VpRef, int*);
 using ColFn = void (*)(ColArgs, Geom, ColWork, BatchRef, const float2*);
+using PairColFn = void (*)(ColArgs, Geom, ColWork, BatchRef, const float2*, CUtensorMap, TmaCoords, CUtensorMap, TmaCoords, int*);
 using TmaColFn = void (*)(ColArgs, Geom, ColWork, BatchRef, const float2*, CUtensorMap, TmaCoords, int*);
 
 // A TMA source description for one column pass: the tensor map over the pass's source array,
@@ -56,7 +58,8 @@ struct XVariant {
   size_t tw = 0, twr = 0;             // offsets of the plan's twiddles and of its reverse's
   size_t tile_smem = 0;
   size_t smem = 0;
-  int ctas = 0;                       // resident CTAs on the device (0: does not fit)
+  int ctas = 0;                       // resident CTAs on the device
+  int state = 0;                      // 0 not set up yet, 1 ready, -1 does not fit
   // precision form: 0 FP32, 1 split FP16 tensor cores, 2 split BF16 tensor cores; the split
   // forms read a per-device constant table (DFT fragments, twiddles) built by build_table
   int prec = 0;
@@ -76,10 +79,12 @@ struct ColVariant {
   std::string name;
   ColFn inv = nullptr, fwd = nullptr;
   TmaColFn inv_tma = nullptr, fwd_tma = nullptr;  // set for TMA-fed variants (inv / fwd unused then)
+  PairColFn inv_pair = nullptr, fwd_pair = nullptr;  // set for column pairs, TMA in and out
   int threads = 0, tx = 0;
   size_t tw = 0;
   size_t smem = 0;
   int ctas_inv = 0, ctas_fwd = 0;
+  int state_inv = 0, state_fwd = 0;  // as XVariant::state
   int pref = 0;  // default of the classes whose bit is set (kDefault*)
 };
 constexpr int kDefaultZinv = 1, kDefaultYinv = 2, kDefaultYfwd = 4, kDefaultZfwd = 8;
@@ -94,7 +99,7 @@ struct PlaneVariant {
   int threads = 0;
   size_t tw = 0;
   size_t smem = 0;
-  int ctas_fwd = 0, ctas_inv = 0;
+  int state_inv = 0, state_fwd = 0;  // as XVariant::state
   int pref = 0;  // default of: bit 0 inverse, bit 1 forward of a single problem; bits 2, 3 of a batch
 };
 
@@ -104,11 +109,12 @@ class OpsBase {
   int setup(const Geom& g);
   // cap: upper bound of the active instances (the grid covers cap instances; the kernels read
   // the actual count from the BatchRef)
-  // tp: the TMA source of this call (nullptr or !ok: a TMA-fed selection falls back to variant 0)
+  // tp, to: the TMA source and destination of this call (nullptr or !ok: a selection that needs it falls back
+  // to variant 0)
   void col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, int cap, cudaStream_t s,
-           const TmaPass* tp = nullptr) const;
+           const TmaPass* tp = nullptr, const TmaPass* to = nullptr) const;
   void x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride, BatchRef br,
-               int cap, unsigned int* vmax, VpRef vp, cudaStream_t s, const TmaPass* tp = nullptr) const;
+               int cap, unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp = nullptr) const;
   // plane passes: forward transforms of nslots planes per kx mode; stage update (a.op) of nf
   // fields and, with inv, their inverse transforms.  cap as in col.
   void plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, int cap, cudaStream_t s) const;
@@ -126,18 +132,17 @@ class OpsBase {
   int n = 0;
   int prec = 0;  // precision form of the x rows (mhd_params.precision)
   int vp = 0;    // volume-penalisation form of the x rows (XVariant::vp)
-  bool vp_capable = false;  // set before setup: prepare the penalty forms too
   int hd = 0;    // set before setup: 1 selects the hydrodynamic x-row form (XVariant::hd)
   // switch the volume-penalisation form; the x-row class falls back to its first variant of the
   // new form (MHD_OK, or MHD_ERR_INVALID when this grid size has none)
   int set_vp(int mode);
-  std::vector<XVariant> xv;
-  std::vector<ColVariant> cv;
+  mutable std::vector<XVariant> xv;  // mutable: variants are set up when first asked for
+  mutable std::vector<ColVariant> cv;
   // plane order (set before setup): the column classes are the plane passes, y_inverse and
   // y_forward being part of z_inverse's and z_forward's launches
   bool planar = false;
   bool batch = false;  // capacity above 1 (set before setup): picks the default plane variants
-  std::vector<PlaneVariant> pv;
+  mutable std::vector<PlaneVariant> pv;
   int sel[kTunedClasses] = {0, 0, 0, 0, 0};  // selected variant of each tuned class
   int variant_count(int cls) const;
   bool variant_ok(int cls, int i) const;
@@ -146,6 +151,11 @@ class OpsBase {
   int select_by_name(int cls, const std::string& name);
 
  protected:
+  bool ready(XVariant& x) const;
+  bool ready(PlaneVariant& v, bool inv) const;
+  bool ready(ColVariant& c, bool inv) const;
+  bool preferred(int cls, int i) const;
+  int sm_count = 0, smem_limit = 0, kxp = 0;
   // plain row transforms (staging of set_physical / get_physical / diagnostics)
   C2RFn c2r = nullptr, c2r_plane = nullptr;
   R2CFn r2c = nullptr, r2c_plane = nullptr;
@@ -207,15 +217,15 @@ class Ops : public OpsBase {
     add_x_form<R, GROUPS, NTI, NTF, MINB, false>();
   }
   // DIRECT: field rows loaded from global memory into registers, no staging copy ("/d")
-  template <class R, int GROUPS, int NTI, int NTF, int MINB, bool DIRECT, bool PLANE = false>
+  template <class R, int GROUPS, int NTI, int NTF, int MINB, bool DIRECT, bool PLANE = false, bool PAIR = false>
   void add_x_form() {
     constexpr int NTS = NTI > NTF ? NTI : NTF;
-    using XC = XCfg<R, NTS, DIRECT>;
+    using XC = XCfg<R, NTS, DIRECT, PAIR>;
     XVariant v;
     v.plane = PLANE;
     v.name = std::string(PLANE ? "xplane:" : "x:") + plan_name<R>() + "/nt" + std::to_string(NTI) + std::to_string(NTF) + "/c" +
-             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (DIRECT && !PLANE ? "/d" : "");
-    v.fn = x_fused_kernel<R, GROUPS, NTI, NTF, MINB, 0, false, DIRECT, PLANE>;
+             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (DIRECT && !PLANE ? "/d" : "") + (PAIR ? "/pair" : "");
+    v.fn = x_fused_kernel<R, GROUPS, NTI, NTF, MINB, 0, false, DIRECT, PLANE, PAIR>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -226,13 +236,13 @@ class Ops : public OpsBase {
   }
 
   // x rows in plane order by TMA tiles, NBUF tiles in flight per CTA
-  template <class R, int NBUF, int MINB, int VPM = 0, bool HDX = false>
+  template <class R, int NBUF, int MINB, int VPM = 0, bool HDX = false, bool PAIR = false>
   void add_x_tile() {
-    using XC = XPlaneCfg<R, NBUF, VPM, HDX>;
+    using XC = XPlaneCfg<R, NBUF, VPM, HDX, PAIR>;
     XVariant v;
     v.name = std::string(HDX ? "xtilehd" : "xtile") + (VPM ? "vp" + std::to_string(VPM) : "") + ":" + plan_name<R>() + "/q" +
-             std::to_string(NBUF) + "/b" + std::to_string(MINB);
-    v.tile_fn = x_plane_kernel<R, NBUF, MINB, VPM, HDX>;
+             std::to_string(NBUF) + "/b" + std::to_string(MINB) + (PAIR ? "/pair" : "");
+    v.tile_fn = x_plane_kernel<R, NBUF, MINB, VPM, HDX, PAIR>;
     v.threads = XC::THREADS;
     v.rpg = XC::ROWS;
     v.tile_smem = XC::SMEM;
@@ -251,14 +261,14 @@ class Ops : public OpsBase {
     add_x_vp_one<R, GROUPS, NTI, MINB, 1, PLANE>();
     add_x_vp_one<R, GROUPS, NTI, MINB, 2, PLANE>();
   }
-  template <class R, int GROUPS, int NTI, int MINB, int VPM, bool PLANE>
+  template <class R, int GROUPS, int NTI, int MINB, int VPM, bool PLANE, bool PAIR = false>
   void add_x_vp_one() {
-    using XC = XCfg<R, NTI, PLANE>;
+    using XC = XCfg<R, NTI, PLANE, PAIR>;
     XVariant v;
     v.plane = PLANE;
     v.name = "xvp" + std::to_string(VPM) + ":" + plan_name<R>() + "/nt" + std::to_string(NTI) + "1/c" +
-             std::to_string(GROUPS) + "/b" + std::to_string(MINB);
-    v.fn = x_fused_kernel<R, GROUPS, NTI, 1, MINB, VPM, false, PLANE, PLANE>;
+             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (PAIR ? "/pair" : "");
+    v.fn = x_fused_kernel<R, GROUPS, NTI, 1, MINB, VPM, false, PLANE, PLANE, PAIR>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -271,14 +281,14 @@ class Ops : public OpsBase {
 
   // x rows of the hydrodynamic form (one transform per exchange round); VPM > 0 adds the
   // velocity penalty fields (VP on hydrodynamics)
-  template <class R, int GROUPS, int MINB, int VPM = 0, bool PLANE = false>
+  template <class R, int GROUPS, int MINB, int VPM = 0, bool PLANE = false, bool PAIR = false>
   void add_x_hd() {
-    using XC = XCfg<R, 1, PLANE>;
+    using XC = XCfg<R, 1, PLANE, PAIR>;
     XVariant v;
     v.plane = PLANE;
     v.name = std::string(VPM ? "xhdvp" + std::to_string(VPM) : "xhd") + ":" + plan_name<R>() + "/nt11/c" +
-             std::to_string(GROUPS) + "/b" + std::to_string(MINB);
-    v.fn = x_fused_kernel<R, GROUPS, 1, 1, MINB, VPM, true, PLANE, PLANE>;
+             std::to_string(GROUPS) + "/b" + std::to_string(MINB) + (PAIR ? "/pair" : "");
+    v.fn = x_fused_kernel<R, GROUPS, 1, 1, MINB, VPM, true, PLANE, PLANE, PAIR>;
     v.threads = GROUPS * XC::TPG;
     v.rpg = XC::RPG;
     v.groups = GROUPS;
@@ -381,6 +391,22 @@ class Ops : public OpsBase {
     c.tx = TX;
     c.smem = sizeof(float2) * NBUF * (size_t)N * TX + NBUF * sizeof(unsigned long long) + 16 +
              (TWS ? sizeof(float2) * PlanTw<C>::SIZE : 0);
+    c.tw = twiddles<C>();
+    c.pref = pref;
+    cv.push_back(c);
+  }
+
+  // column passes on pairs of columns, TMA in and out
+  template <class C, int MINB, int NBUF>
+  void add_col_pair(int pref = 0) {
+    constexpr int TX = 16;  // the tensor maps' boxes: 16 columns
+    ColVariant c;
+    c.name = "colpair:" + plan_name<C>() + "/tx" + std::to_string(TX) + "/b" + std::to_string(MINB) + "/q" + std::to_string(NBUF);
+    c.inv_pair = col_pair_kernel<C, TX, +1, true, false, MINB, NBUF>;
+    c.fwd_pair = col_pair_kernel<C, TX, -1, false, true, MINB, NBUF>;
+    c.threads = TX / 2 * C::G;
+    c.tx = TX;
+    c.smem = sizeof(float2) * NBUF * (size_t)N * TX + NBUF * sizeof(unsigned long long) + 16;
     c.tw = twiddles<C>();
     c.pref = pref;
     cv.push_back(c);

@@ -37,6 +37,57 @@ bool is_inv(int cls) { return cls == KC_ZINV || cls == KC_YINV; }
 
 }  // namespace
 
+// A variant's kernels are set up (attributes, occupancy, tables) when it is first asked for: a handle
+// that runs on its defaults pays for those alone.
+bool OpsBase::ready(XVariant& x) const {
+  if (x.state) return x.state > 0;
+  x.state = -1;
+  const void* fn = x.tile_fn ? (const void*)x.tile_fn : (const void*)x.fn;
+  x.smem = x.tile_fn ? x.tile_smem : sizeof(float2) * (size_t)x.groups * x.group_words(kxp);
+  if ((int)x.smem > smem_limit) return false;
+  if (x.build_table) {
+    if (cudaMalloc(&x.table, x.table_words * sizeof(uint32_t)) != cudaSuccess) {
+      cudaGetLastError();
+      x.table = nullptr;
+      return false;
+    }
+    if (x.build_table(x.table)) return false;
+  }
+  // max_carveout: the whole unified L1 / shared array as shared memory (two CTAs per SM fit only then)
+  if (set_smem(fn, x.smem) ||
+      (x.max_carveout && cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess) ||
+      resident_ctas(fn, x.threads, x.smem, sm_count, &x.ctas) || x.ctas == 0)
+    return false;
+  x.state = 1;
+  return true;
+}
+bool OpsBase::ready(PlaneVariant& v, bool inv) const {
+  int& state = inv ? v.state_inv : v.state_fwd;
+  if (state) return state > 0;
+  state = -1;
+  if ((int)v.smem > smem_limit) return false;
+  int ctas = 0;
+  const void* main = inv ? (const void*)v.inv : (const void*)v.fwd;
+  if (set_smem(main, v.smem) || resident_ctas(main, v.threads, v.smem, sm_count, &ctas) || ctas == 0) return false;
+  if (inv)
+    for (const void* f : {(const void*)v.stage, (const void*)v.stage_gen, (const void*)v.stage_hd})
+      if (f && set_smem(f, v.smem)) return false;
+  state = 1;
+  return true;
+}
+bool OpsBase::ready(ColVariant& c, bool inv) const {
+  int& state = inv ? c.state_inv : c.state_fwd;
+  if (state) return state > 0;
+  state = -1;
+  if ((int)c.smem > smem_limit) return false;
+  const void* f = inv ? (c.inv_pair ? (const void*)c.inv_pair : c.inv_tma ? (const void*)c.inv_tma : (const void*)c.inv)
+                      : (c.fwd_pair ? (const void*)c.fwd_pair : c.fwd_tma ? (const void*)c.fwd_tma : (const void*)c.fwd);
+  int& ctas = inv ? c.ctas_inv : c.ctas_fwd;
+  if (set_smem(f, c.smem) || resident_ctas(f, c.threads, c.smem, sm_count, &ctas) || ctas == 0) return false;
+  state = 1;
+  return true;
+}
+
 int OpsBase::setup(const Geom& g) {
   if (g.kx != kept_kx_of(n) || g.kp != kept_kx_of(n) || g.kn != kept_kn_of(n))
     return report_error(MHD_ERR_INVALID, "kept-mode counts differ from the compiled pass plans");
@@ -49,62 +100,22 @@ int OpsBase::setup(const Geom& g) {
   if (e != cudaSuccess) return report_error(MHD_ERR_OOM, std::string("twiddle tables: ") + cudaGetErrorString(e));
   e = cudaMemcpy(tw_dev, tw_host.data(), tw_host.size() * sizeof(float2), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return report_error(MHD_ERR_CUDA, std::string("twiddle upload: ") + cudaGetErrorString(e));
-  for (auto& x : xv) {
-    const void* fn = x.tile_fn ? (const void*)x.tile_fn : (const void*)x.fn;
-    x.smem = x.tile_fn ? x.tile_smem : sizeof(float2) * (size_t)x.groups * x.group_words(g.kxp);
-    x.ctas = 0;
-    if (x.prec != prec || (int)x.smem > smem_max) continue;  // only this problem's precision form
-    if (x.vp && !vp_capable) continue;                       // penalty forms only with VP on
-    if (x.hd != hd) continue;                                // this problem's field set only
-    if (x.plane != planar) continue;                         // this problem's layout only
-    if (x.build_table) {
-      e = cudaMalloc(&x.table, x.table_words * sizeof(uint32_t));
-      if (e != cudaSuccess) return report_error(MHD_ERR_OOM, std::string("tensor-core tables: ") + cudaGetErrorString(e));
-      if (x.build_table(x.table)) return report_error(MHD_ERR_CUDA, "building the tensor-core DFT tables failed");
-    }
-    if ((rc = set_smem(fn, x.smem))) return rc;
-    if (x.max_carveout) {
-      // the whole unified L1 / shared array as shared memory: two CTAs per SM fit only then
-      e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-      if (e != cudaSuccess) return report_error(MHD_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-    }
-    if ((rc = resident_ctas(fn, x.threads, x.smem, sms, &x.ctas))) return rc;
-  }
-  for (auto& v : pv) {
-    v.ctas_fwd = v.ctas_inv = 0;
-    if (!planar || (int)v.smem > smem_max) continue;
-    for (const void* f : {(const void*)v.fwd, (const void*)v.inv, (const void*)v.stage, (const void*)v.stage_gen, (const void*)v.stage_hd})
-      if (f && (rc = set_smem(f, v.smem))) return rc;
-    if ((rc = resident_ctas((const void*)v.fwd, v.threads, v.smem, sms, &v.ctas_fwd))) return rc;
-    if ((rc = resident_ctas((const void*)v.inv, v.threads, v.smem, sms, &v.ctas_inv))) return rc;
-  }
-  for (auto& c : cv) {
-    c.ctas_inv = c.ctas_fwd = 0;
-    if (planar) continue;
-    if ((int)c.smem > smem_max) continue;
-    const void* fi = c.inv_tma ? (const void*)c.inv_tma : (const void*)c.inv;
-    const void* ff = c.fwd_tma ? (const void*)c.fwd_tma : (const void*)c.fwd;
-    if ((rc = set_smem(fi, c.smem))) return rc;
-    if ((rc = set_smem(ff, c.smem))) return rc;
-    if ((rc = resident_ctas(fi, c.threads, c.smem, sms, &c.ctas_inv))) return rc;
-    if ((rc = resident_ctas(ff, c.threads, c.smem, sms, &c.ctas_fwd))) return rc;
-  }
-  if (!cv.empty() && cv[0].inv_tma) return report_error(MHD_ERR_INVALID, "the default column variant must not be TMA-fed");
+  sm_count = sms;
+  smem_limit = smem_max;
+  kxp = g.kxp;
+  if (!cv.empty() && (cv[0].inv_tma || cv[0].inv_pair)) return report_error(MHD_ERR_INVALID, "the default column variant must not be TMA-fed");
   if ((rc = set_smem(planar ? (const void*)c2r_plane : (const void*)c2r, row_smem))) return rc;
   if ((rc = set_smem(planar ? (const void*)r2c_plane : (const void*)r2c, row_smem))) return rc;
+  // the single-field transforms and a missing tensor map fall back to the first column variant
+  if (!planar && (cv.empty() || !ready(cv[0], true) || !ready(cv[0], false)))
+    return report_error(MHD_ERR_CUDA, "no pass-kernel variant fits on this device");
   // the default of each class is its first variant that fits on this device and names the class as its
   // own, else the first that fits
   for (int cls = 0; cls < kTunedClasses; ++cls) {
     int i = 0;
-    while (i < variant_count(cls) && !variant_ok(cls, i)) ++i;
-    if (planar && plane_cls(cls))  // or the first that is meant for this class and capacity
-      for (int j = i; j < variant_count(cls); ++j)
-        if (variant_ok(cls, j) && (pv[j].pref >> (is_inv(cls) ? 0 : 1) >> (batch ? 2 : 0) & 1)) { i = j; break; }
-    if (!planar && is_col(cls)) {
-      const int bit = cls == KC_ZINV ? kDefaultZinv : cls == KC_YINV ? kDefaultYinv : cls == KC_YFWD ? kDefaultYfwd : kDefaultZfwd;
-      for (int j = i; j < variant_count(cls); ++j)
-        if (variant_ok(cls, j) && (cv[j].pref & bit)) { i = j; break; }
-    }
+    while (i < variant_count(cls) && !(preferred(cls, i) && variant_ok(cls, i))) ++i;
+    if (i == variant_count(cls))
+      for (i = 0; i < variant_count(cls) && !variant_ok(cls, i);) ++i;
     if (i == variant_count(cls))
       return report_error(cls == KC_XFUSED && prec ? MHD_ERR_INVALID : MHD_ERR_CUDA,
                           cls == KC_XFUSED && prec ? "no x-row kernel of this precision form for this grid size"
@@ -112,6 +123,13 @@ int OpsBase::setup(const Geom& g) {
     sel[cls] = i;
   }
   return MHD_OK;
+}
+
+// whether a variant names the class (and, in plane order, the capacity) as its own
+bool OpsBase::preferred(int cls, int i) const {
+  if (cls == KC_XFUSED) return true;  // one default for all capacities: a slot's results equal a single problem's bit for bit
+  if (planar) return !plane_cls(cls) || (pv[i].pref >> (is_inv(cls) ? 0 : 1) >> (batch ? 2 : 0) & 1);
+  return cv[i].pref & (cls == KC_ZINV ? kDefaultZinv : cls == KC_YINV ? kDefaultYinv : cls == KC_YFWD ? kDefaultYfwd : kDefaultZfwd);
 }
 
 int OpsBase::set_vp(int mode) {
@@ -133,10 +151,10 @@ int OpsBase::variant_count(int cls) const {
 
 bool OpsBase::variant_ok(int cls, int i) const {
   if (i < 0 || i >= variant_count(cls)) return false;
-  if (cls == KC_XFUSED)
-    return xv[i].ctas > 0 && xv[i].prec == prec && xv[i].vp == vp && xv[i].hd == hd && xv[i].plane == planar;
-  if (planar) return !plane_cls(cls) || (is_inv(cls) ? pv[i].ctas_inv : pv[i].ctas_fwd) > 0;
-  return is_inv(cls) ? cv[i].ctas_inv > 0 : cv[i].ctas_fwd > 0;
+  if (cls == KC_XFUSED)  // this problem's precision, penalty form, field set and layout only
+    return xv[i].prec == prec && xv[i].vp == vp && xv[i].hd == hd && xv[i].plane == planar && ready(xv[i]);
+  if (planar) return !plane_cls(cls) || ready(pv[i], is_inv(cls));
+  return ready(cv[i], is_inv(cls));
 }
 
 std::string OpsBase::variant_name(int cls, int i) const {
@@ -161,23 +179,23 @@ int OpsBase::select_by_name(int cls, const std::string& name) {
 }
 
 void OpsBase::col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, int cap,
-                  cudaStream_t s, const TmaPass* tp) const {
-  const bool tma_sel = cv[sel[cls]].inv_tma != nullptr;
-  const ColVariant& c = (tma_sel && !(tp && tp->ok)) ? cv[0] : cv[sel[cls]];
+                  cudaStream_t s, const TmaPass* tp, const TmaPass* to) const {
+  const ColVariant& sv = cv[sel[cls]];
+  const bool in = tp && tp->ok, out = to && to->ok;
+  const ColVariant& c = (sv.inv_tma && !in) || (sv.inv_pair && !(in && out)) ? cv[0] : sv;
   const bool inv = is_inv(cls);
-  if (c.inv_tma) {
-    const ColWork w{(g.kx + c.tx - 1) / c.tx, outer, nf, inv ? g.k2 : n};
-    const long long total = (long long)cap * w.tiles_x * w.outer * w.nf;
-    const int ctas = inv ? c.ctas_inv : c.ctas_fwd;
-    const int grid = (int)(total < ctas ? total : ctas);
-    const TmaColFn f = inv ? c.inv_tma : c.fwd_tma;
-    f<<<grid, c.threads, c.smem, s>>>(a, g, w, br, tw_dev + c.tw, tp->map, tp->tc, tp->err);
-    return;
-  }
   const ColWork w{(g.kx + c.tx - 1) / c.tx, outer, nf, inv ? g.k2 : n};
   const long long total = (long long)cap * w.tiles_x * w.outer * w.nf;
   const int ctas = inv ? c.ctas_inv : c.ctas_fwd;
   const int grid = (int)(total < ctas ? total : ctas);
+  if (c.inv_pair) {
+    (inv ? c.inv_pair : c.fwd_pair)<<<grid, c.threads, c.smem, s>>>(a, g, w, br, tw_dev + c.tw, tp->map, tp->tc, to->map, to->tc, tp->err);
+    return;
+  }
+  if (c.inv_tma) {
+    (inv ? c.inv_tma : c.fwd_tma)<<<grid, c.threads, c.smem, s>>>(a, g, w, br, tw_dev + c.tw, tp->map, tp->tc, tp->err);
+    return;
+  }
   const ColFn f = inv ? c.inv : c.fwd;
   f<<<grid, c.threads, c.smem, s>>>(a, g, w, br, tw_dev + c.tw);
 }
@@ -200,7 +218,7 @@ void OpsBase::plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, i
 }
 
 void OpsBase::x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride,
-                      BatchRef br, int cap, unsigned int* vmax, VpRef vp, cudaStream_t s, const TmaPass* tp) const {
+                      BatchRef br, int cap, unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp) const {
   const XVariant* sv = &xv[sel[KC_XFUSED]];
   if (sv->tile_fn && !(tp && tp->ok))  // no tensor map: the first variant of this form without one
     for (size_t i = 0; i < xv.size(); ++i)
@@ -217,7 +235,7 @@ void OpsBase::x_fused(float2* pool, const Geom& g, long long rowstride, long lon
   const int grid = (int)(need < x.ctas ? need : x.ctas);
   const float2* t1 = x.table ? reinterpret_cast<const float2*>(x.table) : tw_dev + x.tw;
   const float2* t2 = x.table ? nullptr : tw_dev + x.twr;
-  x.fn<<<grid, x.threads, x.smem, s>>>(pool, g, rowstride, slot, istride, br, t1, t2, vmax, vp);
+  x.fn<<<grid, x.threads, x.smem, s>>>(pool, g, rowstride, slot, istride, br, t1, t2, vmax, vp, err);
 }
 
 int OpsBase::x_device_error() const {

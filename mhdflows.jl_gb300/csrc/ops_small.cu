@@ -22,8 +22,8 @@ OpsBase* make_ops_32() {
   using R = Plan<32, 4, 8, 4>;
   auto* o = new Ops<32>();
   o->add_plane<R, 128, 6>();                     // inverse 7.3, 12.9; forward 6.1, 12.0
-  o->add_x_form<R, 1, 1, 1, 16, true, true>();
-  o->add_x_tile<R, 1, 7>();
+  o->add_x_tile<R, 1, 8, 0, false, true>();      // 7.9, 16.5
+  o->add_x_form<R, 1, 1, 1, 16, true, true>();   // 8.1, 20.5
   o->add_x_vp<R, 1, 1, 16, true>();
   o->add_x_hd<R, 1, 16, 0, true>();
   o->add_x_hdvp<R, 1, 16, true>();
@@ -36,7 +36,7 @@ OpsBase* make_ops_48() {
   auto* o = new Ops<48>();
   o->add_plane<R, 192, 1>(1 | 2);                // inverse 9.2, 39.7; forward 7.7, 22.4
   o->add_plane<R, 128, 6>(4 | 8);                // inverse 10.5, 28.6; forward 8.0, 20.3
-  o->add_x_tile<R, 1, 5>();
+  o->add_x_tile<R, 1, 5, 0, false, true>();      // 9.6, 34.7 (one at a time 10.0, 42.8)
   o->add_x_form<R, 1, 1, 1, 8, true, true>();
   o->add_x_tile<R, 1, 4, 1>();
   o->add_x_tile<R, 1, 4, 2>();
@@ -55,7 +55,7 @@ OpsBase* make_ops_64() {
   auto* o = new Ops<64>();
   o->add_plane<R, 512, 1>(1);                    // inverse 9.9, 54.1; forward 9.0, 28.7
   o->add_plane<R, 192, 5>(2 | 4 | 8);            // inverse 13.6, 42.2; forward 8.3, 24.4
-  o->add_x_tile<R, 2, 3>();
+  o->add_x_tile<R, 2, 3, 0, false, true>();      // 9.7, 33.8 (one at a time 10.2, 38.3)
   o->add_x_form<R, 1, 1, 1, 16, true, true>();
   o->add_x_tile<R, 1, 3, 1>();
   o->add_x_tile<R, 1, 3, 2>();

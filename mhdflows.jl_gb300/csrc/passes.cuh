@@ -11,6 +11,7 @@
 #include <cuda.h>
 
 #include "fft_core.cuh"
+#include "fft_pair.cuh"
 
 namespace mhdgb {
 
@@ -342,6 +343,12 @@ __global__ void __launch_bounds__(TX * P0::G, MINB)
 // timeout the kernel records the failure in *err, stops taking tiles, waits (bounded again) for
 // the copies it issued and returns.
 // ------------------------------------------------------------------------------------------
+__device__ __forceinline__ void bulk_load(unsigned int dst, const void* src, unsigned int bytes, unsigned int bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+               "r"(bytes), "r"(bar)
+               : "memory");
+}
+
 struct TmaCoords {
   int rowdim, odim, fdim, idim;  // tensor-map dimensions of the transformed axis, outer index, field, slot
   int rb;                        // rows per box
@@ -708,19 +715,24 @@ __device__ __forceinline__ void x_vmax(const float2 (&v)[3][V], unsigned int* vm
 // Products: Dxz = (bx^2-ux^2)-(bz^2-uz^2), Dyz = (by^2-uy^2)-(bz^2-uz^2), Txy, Txz, Tyz with
 // Tij = bi*bj - ui*uj, and Axy, Axz, Ayz with Aij = ui*bj - bi*uj.
 // A row group is RPG = max(1, 32/G) consecutive rows handled by one warp (G <= 32) or one row
-// handled by G/32 warps.  Groups are persistent: while a group transforms its rows, cp.async
-// brings the six field rows of its next rows into the other half of a double buffer.
+// handled by G/32 warps.  Groups are persistent: while a group transforms its rows, bulk copies
+// bring the six field rows of its next rows into the other half of a double buffer.
 // DIRECT: the field rows are read from global memory straight into registers (coalesced across
 // the lanes of a row), with no staging copy in shared memory.
-template <class P, int NTS = 1, bool DIRECT = false>
+// PAIR: the exchange space holds a pair of transforms.
+template <class P, int NTS = 1, bool DIRECT = false, bool PAIR = false>
 struct XCfg {
   static constexpr int G = P::G;
   static constexpr int RPG = G >= 32 ? 1 : 32 / G;        // rows per group
   static constexpr int TPG = G >= 32 ? G : 32;            // threads per group
-  static constexpr int TS = RowCfg<P>::TS;                // exchange words per transform
+  static constexpr int PW = PairRow<P>::WORDS > PairRow<typename Reverse<P>::type>::WORDS
+                                ? PairRow<P>::WORDS
+                                : PairRow<typename Reverse<P>::type>::WORDS;
+  static constexpr int TS = PAIR && 2 * PW > RowCfg<P>::TS ? 2 * PW : RowCfg<P>::TS;  // exchange words per transform
   static __host__ __device__ int stage_words(int kxp) { return DIRECT ? 0 : RPG * 6 * kxp; }
-  // two staging buffers of the six field rows, then NTS exchange buffers per row
-  static __host__ __device__ int group_words(int kxp) { return 2 * stage_words(kxp) + RPG * NTS * TS; }
+  // two staging buffers of the six field rows, then NTS exchange buffers per row, then the staging
+  // buffers' mbarriers and the group's abort flag
+  static __host__ __device__ int group_words(int kxp) { return 2 * stage_words(kxp) + RPG * NTS * TS + (DIRECT ? 0 : 4); }
 };
 
 // Variants (chosen per grid size by the autotuner): NTI inverse transforms (1 or 3) and NTF
@@ -735,14 +747,16 @@ struct XCfg {
 // sixth slot written is zero).
 // PLANE: the rows lie in plane order (kx modes n^2 apart, rows of consecutive y adjacent: rowstride
 // 1, slot stride Kx n^2), read straight into registers (DIRECT).
+// PAIR: the first two inverse transforms run as a pair (fft_pair.cuh), and so do the forward ones.
 template <class P, int GROUPS, int NTI, int NTF, int MINB, int VPM = 0, bool HDX = false, bool DIRECT = false,
-          bool PLANE = false>
+          bool PLANE = false, bool PAIR = false>
 __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     x_fused_kernel(float2* pool, Geom geo, long long rowstride, long long slot, long long istride, BatchRef br,
-                   const float2* __restrict__ tw, const float2* __restrict__ twr, unsigned int* vmax, VpRef vp) {
+                   const float2* __restrict__ tw, const float2* __restrict__ twr, unsigned int* vmax, VpRef vp, int* err) {
   using PR = typename Reverse<P>::type;
   constexpr int NTS = NTI > NTF ? NTI : NTF;
-  using XC = XCfg<P, NTS, DIRECT>;
+  using XC = XCfg<P, NTS, DIRECT, PAIR>;
+  static_assert(!PAIR || (NTI == 1 && NTF == 1 && P::G <= 32), "pairs need the row inside one warp");
   static_assert(NTI == 1 || NTI == 3, "inverse transforms go one or three at a time");
   static_assert(NTF == 1 || NTF == 2 || NTF == 4, "forward transforms go one, two or four at a time");
   static_assert(NTF == 1 || P::G <= 32, "batched forward transforms need the row inside one warp");
@@ -768,7 +782,14 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   const RowSync<G> sync{1 + grp};
   constexpr int GPI = N * N / RPG;  // row groups per instance
   const long long ngroups = (long long)(*br.count) * GPI;
-  const int chunks_row = (HDX ? 3 : 6) * kxp / 2;  // 16-byte chunks of the contiguous field rows (slot == kxp)
+  const unsigned int row_bytes = (HDX ? 3 : 6) * kxp * 8;  // the contiguous field rows (slot == kxp)
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(gs + 2 * sw + RPG * NTS * TS);
+  volatile int& abort_flag = *reinterpret_cast<volatile int*>(bars + 2);
+  if (!DIRECT && gt == 0) {
+    abort_flag = 0;
+    for (int b = 0; b < 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[b])) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   // first row of row group q, inside its instance's rowbuf.  Groups are taken from the last one
   // down: the y pass before this kernel wrote the last z planes last (still in L2), and the y
   // pass after it reads the first z planes first (written here last).
@@ -778,33 +799,39 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     return pool + br.slot(inst) * istride + (q - (long long)inst * GPI) * RPG * rowstride;
   };
 
-  // rows q*RPG .. q*RPG+RPG-1 -> dst (each row's six fields contiguous)
-  auto prefetch = [&](long long q, float2* dst) {
+  // rows q*RPG .. q*RPG+RPG-1 -> staging buffer b (each row's six fields contiguous): one bulk copy per
+  // row, completing on the buffer's mbarrier.  (16-byte cp.async by the lanes took 33 of 680 wavefronts
+  // per 256-point row on the L1 data pipe, which binds this kernel, and their addresses.)
+  auto prefetch = [&](long long q, int b) {
+    if (gt != 0) return;
     const float2* src = group_rows(q);
-    for (int c = gt; c < RPG * chunks_row; c += TPG) {
-      const int r = RPG == 1 ? 0 : c / chunks_row;
-      const int cc = RPG == 1 ? c : c - r * chunks_row;
-      cp_async16(dst + r * 6 * kxp + 2 * cc, src + r * rowstride + 2 * cc);
-    }
+    const unsigned int bar = smem_u32(&bars[b]);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier generic reads of the buffer
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(RPG * row_bytes) : "memory");
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) bulk_load(smem_u32(gs + b * sw + r * 6 * kxp), src + r * rowstride, row_bytes, bar);
   };
 
   long long q = (long long)blockIdx.x * GROUPS + grp;
   const long long qstep = (long long)gridDim.x * GROUPS;
-  if (!DIRECT && q < ngroups) prefetch(q, gs);
-  cp_async_commit();
-  for (int it = 0; q < ngroups; q += qstep, ++it) {
+  if (!DIRECT && q < ngroups) prefetch(q, 0);
+  int it = 0;
+  for (; q < ngroups; q += qstep, ++it) {
     const float2* rin;
     if constexpr (DIRECT) {
       // this row's own slots; every lane loads its inputs before any lane
       // stores an output over them (the stores follow the transforms)
       rin = group_rows(q) + rr * rowstride;
     } else {
-      const float2* cur = gs + (it & 1) * sw;
-      if (q + qstep < ngroups) prefetch(q + qstep, gs + ((it + 1) & 1) * sw);
-      cp_async_commit();
-      cp_async_wait<1>();
+      if (it == 0) sync();  // the barriers are initialised
+      if (q + qstep < ngroups) prefetch(q + qstep, (it + 1) & 1);
+      if (!mbar_wait(smem_u32(&bars[it & 1]), (unsigned int)((it >> 1) & 1))) {
+        atomicExch(err, 1);
+        abort_flag = 1;
+      }
       sync();
-      rin = cur + rr * 6 * kxp;
+      if (abort_flag) break;
+      rin = gs + (it & 1) * sw + rr * 6 * kxp;
     }
     const long long rs = PLANE ? slot : (long long)kxp;  // field stride of the row's inputs
     float2 v[3][V];
@@ -814,7 +841,22 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       if (HDX && t == 1) load_herm_pair<P, KX, true>(v[t], f1, f2, g);
       else load_herm_pair<P, KX>(v[t], f1, f2, g);
     }
-    if constexpr (NTI == 3) {
+    if constexpr (PAIR) {
+      C2 z[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i) z[i] = C2{make_float2(v[0][i].x, v[1][i].x), make_float2(v[0][i].y, v[1][i].y)};
+      fft_run_pair<P, +1>(z, reinterpret_cast<float4*>(sb), g, tw, sync);
+      sync();
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        v[0][i] = make_float2(z[i].re.x, z[i].im.x);
+        v[1][i] = make_float2(z[i].re.y, z[i].im.y);
+      }
+      if constexpr (!HDX) {
+        fft_run<P, +1, 1, TS, 1, false>(reinterpret_cast<float2(&)[1][V]>(v[2]), sb, 0, g, tw, sync);
+        sync();
+      }
+    } else if constexpr (NTI == 3) {
       fft_run<P, +1, 3, TS, 1, false>(v, sb, 0, g, tw, sync);
       sync();
     } else {
@@ -854,6 +896,38 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     }
     // NTF product pairs at a time: the six fields stay live, each pair is formed just before its
     // forward transform (fewer live registers than all eight products at once)
+    if constexpr (PAIR) {
+      auto put_rows = [&](const float2(&w)[V], int t) {
+        split_shfl<PR, KX>(w, g, (threadIdx.x & 31) - g, [&](int k, float2 a, float2 b) {
+          float2* o = rowp + (2 * t) * slot + k * XS;
+          o[0] = a;
+          o[slot] = b;
+        });
+      };
+#pragma unroll
+      for (int t0 = 0; t0 < NPAIR; t0 += 2) {
+        float2 w[2][V];
+        x_pair<P, VPM, HDX>(w[0], t0, v, chi, wrow, vp.cs, g);
+        if (t0 + 1 < NPAIR) {
+          x_pair<P, VPM, HDX>(w[1], t0 + 1, v, chi, wrow, vp.cs, g);
+          C2 z[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) z[i] = C2{make_float2(w[0][i].x, w[1][i].x), make_float2(w[0][i].y, w[1][i].y)};
+          fft_run_pair<PR, -1>(z, reinterpret_cast<float4*>(sb), g, twr, sync);
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            w[0][i] = make_float2(z[i].re.x, z[i].im.x);
+            w[1][i] = make_float2(z[i].re.y, z[i].im.y);
+          }
+          put_rows(w[0], t0);
+          put_rows(w[1], t0 + 1);
+        } else {
+          fft_run<PR, -1, 1, TS, 1>(reinterpret_cast<float2(&)[1][V]>(w[0]), sb, 0, g, twr, sync);
+          put_rows(w[0], t0);
+        }
+        sync();  // the next transform's first exchange overwrites sb
+      }
+    } else
 #pragma unroll
     for (int t0 = 0; t0 < NPAIR; t0 += NTF) {
       float2 w[NTF][V];
@@ -884,7 +958,11 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       }
     }
   }
-  cp_async_wait<0>();
+  // after an abort: let the copies this group issued and did not consume land before exiting
+  if (!DIRECT && gt == 0 && q < ngroups && abort_flag) {
+    (void)mbar_wait(smem_u32(&bars[it & 1]), (unsigned int)((it >> 1) & 1));
+    if (q + qstep < ngroups) (void)mbar_wait(smem_u32(&bars[(it + 1) & 1]), (unsigned int)(((it + 1) >> 1) & 1));
+  }
 }
 
 // Plain c2r of row pairs: spectral rows (2q, 2q+1) -> physical rows times scale (1/n^3: the

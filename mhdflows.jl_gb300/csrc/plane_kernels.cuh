@@ -12,14 +12,13 @@
 //   state    S[f][kx][kz'][ky']   ky' rows padded to k2p (compact fields of stride fs)
 //   planes   R[slot][kx][z][y]    between the plane passes and the x rows (in rowbuf)
 //   products P[slot][kx][kz'][ky'] (in colbuf), as the state
-// Both passes touch whole contiguous planes, and the x rows, which take 2 to 8 consecutive y at a
-// time, touch 16- to 64-byte pieces of them.
+// The x rows take tiles of 16 consecutive y of every kx mode and slot by TMA (x_plane_kernel).
 #pragma once
 #include "stage_math.cuh"
 
 namespace mhdgb {
 
-// Largest grid size with plane passes: at 128 a plane takes 156 KB of a CTA's shared memory.
+// Largest grid size with plane passes: at 128 a plane takes 88 KB of shared memory, at 256 it would take 350.
 constexpr int kPlaneMax = 128;
 // Grid sizes whose stage update is fused with the inverse plane pass (plane_stage_kernel).
 __host__ __device__ constexpr bool plane_fused(int n) { return n <= 64; }
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_stage_kernel(RkArgs a, Pl
 // a 32-byte piece per kx mode and warp at G = 8 (measured: 96^3 x 8 boxes 145 us against 95 us for
 // contiguous rows), with tiles every piece is a full 128-byte line.
 // ------------------------------------------------------------------------------------------
-template <class P, int NBUF, int VPM, bool HDX>
+template <class P, int NBUF, int VPM, bool HDX, bool PAIR>
 struct XPlaneCfg {
   static constexpr int N = P::N, G = P::G, ROWS = 16, THREADS = ROWS * G;
   static constexpr int KX = kept_kx_of(N);
@@ -406,7 +405,7 @@ struct XPlaneCfg {
   static constexpr int NSLOT = 2 * NPAIR > NIN ? 2 * NPAIR : NIN;
   static constexpr int SLOTB = (KX + 7) / 8 * 1024;    // bytes of a slot: kx rows of 128 bytes, whole swizzle periods
   static constexpr int TILEB = NSLOT * SLOTB;
-  static constexpr int TS = RowCfg<P>::TS;
+  static constexpr int TS = XCfg<P, 1, true, PAIR>::TS;
   static constexpr size_t SMEM = 1024 + (size_t)NBUF * TILEB + sizeof(float2) * ROWS * TS + 32;
   static_assert(N % ROWS == 0 && NBUF >= 1 && NBUF <= 2, "whole tiles, one or two buffers");
 };
@@ -423,12 +422,13 @@ __device__ __forceinline__ void tma_store4(const void* map, int c0, int c1, int 
                : "memory");
 }
 
-template <class P, int NBUF, int MINB, int VPM = 0, bool HDX = false>
+// PAIR: transforms in pairs as in x_fused_kernel.
+template <class P, int NBUF, int MINB, int VPM = 0, bool HDX = false, bool PAIR = false>
 __global__ void __launch_bounds__(16 * P::G, MINB)
     x_plane_kernel(const __grid_constant__ CUtensorMap map, int* err, BatchRef br, const float2* __restrict__ tw,
                    const float2* __restrict__ twr, unsigned int* vmax, VpRef vp) {
   using PR = typename Reverse<P>::type;
-  using C = XPlaneCfg<P, NBUF, VPM, HDX>;
+  using C = XPlaneCfg<P, NBUF, VPM, HDX, PAIR>;
   constexpr int N = P::N, G = P::G, V = P::V, KX = C::KX, TS = C::TS;
   constexpr int NINV = HDX ? 2 : 3;
   extern __shared__ unsigned char xsm[];
@@ -486,8 +486,20 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
       if (HDX && p == 1) load_herm_pair<P, KX, true>(v[p], f1, f2, g);
       else load_herm_pair<P, KX>(v[p], f1, f2, g);
     }
+    if constexpr (PAIR) {
+      C2 c[V];
 #pragma unroll
-    for (int p = 0; p < NINV; ++p) {
+      for (int i = 0; i < V; ++i) c[i] = C2{make_float2(v[0][i].x, v[1][i].x), make_float2(v[0][i].y, v[1][i].y)};
+      fft_run_pair<P, +1>(c, reinterpret_cast<float4*>(sb), g, tw, sync);
+      sync();
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        v[0][i] = make_float2(c[i].re.x, c[i].im.x);
+        v[1][i] = make_float2(c[i].re.y, c[i].im.y);
+      }
+    }
+#pragma unroll
+    for (int p = PAIR ? 2 : 0; p < NINV; ++p) {
       fft_run<P, +1, 1, TS, 1, false>(reinterpret_cast<float2(&)[1][V]>(v[p]), sb, 0, g, tw, sync);
       sync();
     }
@@ -512,16 +524,34 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
 #pragma unroll
         for (int e = 0; e < P::RF; ++e) chi[d * P::RF + e] = __ldg(crow + g + G * d + P::LF * e);
     }
-#pragma unroll
-    for (int p = 0; p < C::NPAIR; ++p) {
-      float2 w[1][V];
-      x_pair<P, VPM, HDX>(w[0], p, v, chi, wrow, vp.cs, g);
-      fft_run<PR, -1, 1, TS, 1>(w, sb, 0, g, twr, sync);
-      // outputs over the row's own elements: its inputs are in registers, other rows' are elsewhere
-      split_shfl<PR, KX>(w[0], g, (threadIdx.x & 31) - g, [&](int k, float2 a, float2 c) {
+    // outputs over the row's own elements: its inputs are in registers, other rows' are elsewhere
+    auto put_rows = [&](const float2(&w)[V], int p) {
+      split_shfl<PR, KX>(w, g, (threadIdx.x & 31) - g, [&](int k, float2 a, float2 c) {
         *at(2 * p, k) = a;
         *at(2 * p + 1, k) = c;
       });
+    };
+#pragma unroll
+    for (int p = 0; p < C::NPAIR; p += PAIR ? 2 : 1) {
+      float2 w[2][V];
+      x_pair<P, VPM, HDX>(w[0], p, v, chi, wrow, vp.cs, g);
+      if (PAIR && p + 1 < C::NPAIR) {
+        x_pair<P, VPM, HDX>(w[1], p + 1, v, chi, wrow, vp.cs, g);
+        C2 c[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) c[i] = C2{make_float2(w[0][i].x, w[1][i].x), make_float2(w[0][i].y, w[1][i].y)};
+        fft_run_pair<PR, -1>(c, reinterpret_cast<float4*>(sb), g, twr, sync);
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+          w[0][i] = make_float2(c[i].re.x, c[i].im.x);
+          w[1][i] = make_float2(c[i].re.y, c[i].im.y);
+        }
+        put_rows(w[0], p);
+        put_rows(w[1], p + 1);
+      } else {
+        fft_run<PR, -1, 1, TS, 1>(reinterpret_cast<float2(&)[1][V]>(w[0]), sb, 0, g, twr, sync);
+        put_rows(w[0], p);
+      }
       sync();  // the next transform's first exchange overwrites sb
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

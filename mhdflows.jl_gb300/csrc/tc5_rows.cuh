@@ -233,7 +233,7 @@ __device__ __forceinline__ float2 tc5_herm(const float2* f1, const float2* f2, i
 template <int N>
 __global__ void __launch_bounds__(128, 2)
     x_fused_tc5_kernel(float2* pool, Geom geo, long long rowstride, long long slot, long long istride, BatchRef br,
-                       const float2* tw, const float2* /*twr*/, unsigned int* vmax, VpRef /*vp*/) {
+                       const float2* tw, const float2* /*twr*/, unsigned int* vmax, VpRef /*vp*/, int* /*err*/) {
   static_assert(N == 256, "two 16-point stages: n = 256");
   constexpr int KX = kept_kx_of(N), R = Tc5Layout::TILE_ROWS;
   using L = Tc5Layout;
