@@ -66,3 +66,21 @@ def test_steps(pkg, mo, n, scheme):
     for _ in range(2):
         st.stepforward(ref)
     assert mo.rel_l2(got, ref, g.retained_mask()) < TOL
+
+
+@pytest.mark.parametrize("n,scheme,cfl", [(16, "RK4", False), (32, "LSRK4", True), (48, "RK4", True), (64, "LSRK4", False)])
+def test_chained_steps_equal_single_ones(pkg, mo, n, scheme, cfl):
+    """One call of many steps runs on graphs of several chained steps, single calls on the graph of
+    one: the states, clocks and forcing draws agree bit for bit."""
+    got = []
+    for calls in ((100,), (1,) * 100):
+        _, _, prob, _ = _problem(pkg, mo, n, "mhd", scheme, dt=1e-4)
+        with prob:
+            pkg.SetUpFk(prob, P=1e-6, seed=5)
+            if cfl:
+                pkg._lib.check(prob._lib.mhd_set_cfl(prob.handle, 1, 0.2))
+            for k in calls:
+                pkg.stepforward(prob, k)
+            got.append((prob.sol_c(), prob.clock.t, prob.clock.step))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert got[0][1:] == got[1][1:]
