@@ -328,6 +328,61 @@ struct Reverse<Plan<N, G, R0, R1, 1>> { using type = Plan<N, G, R1, R0, 1>; };
 template <int N, int G, int R0, int R1, int R2>
 struct Reverse<Plan<N, G, R0, R1, R2>> { using type = Plan<N, G, R2, R1, R0>; };
 
+// A row of 2 H::N points as two interleaved half transforms: even points on the even lanes, odd points
+// on the odd ones, each half a two-stage transform with one shared-memory exchange, joined by a
+// radix-2 step between lanes g and g ^ 1 (two shuffles per value).  Index conventions on the spectral
+// side are Plan's with G = 2 H::G lanes; on the physical side register i of lane g holds point
+// phys_x(g, i), for an inverse's outputs and for the inputs of the reversed plan's forward alike.
+// Where Plan needs three stages (96 = 12 x 4 x 2) this trades the second exchange (four data-pipe
+// wavefronts per 32 values) for the shuffles (two) and a shorter chain: x rows of eight 96^3 boxes 93 ->
+// 83 us.  Where Plan has two wide stages it is slower (256: 2 x 16 x 8 at 199 us against 16 x 16 at 160),
+// and at 512 (2 x 16 x 16, 1655 us against 8 x 8 x 8 at 1560) the wide halves leave too few warps.
+template <class H_>
+struct Split2 {
+  using H = H_;
+  static_assert(H::STAGES == 2, "two-stage halves");
+  static constexpr int N = 2 * H::N, G = 2 * H::G, V = H::V;
+  static constexpr int R0 = H::R0, R1 = H::R1, R2 = 1, RF = H::RF, STAGES = 2;
+  static constexpr int LI = 2 * H::LI, LF = 2 * H::LF, DI = H::DI, DF = H::DF;
+};
+template <class H>
+struct Reverse<Split2<H>> { using type = Split2<typename Reverse<H>::type>; };
+
+template <class P>
+struct IsSplit { static constexpr bool value = false; };
+template <class H>
+struct IsSplit<Split2<H>> { static constexpr bool value = true; };
+
+// Physical point of register i of lane g between an inverse and a forward transform.
+template <class P>
+__host__ __device__ __forceinline__ constexpr int phys_x(int g, int i) {
+  if constexpr (IsSplit<P>::value)
+    return g / 2 + P::H::G * (i / P::RF) + P::H::LF * (i % P::RF) + P::H::N * (g % 2);
+  else
+    return g + P::G * (i / P::RF) + P::LF * (i % P::RF);
+}
+
+// Half plan with an odd exchange stride, and the offsets of the halves and rows in shared memory that
+// keep the lanes of a half-warp (8-byte words; quarter-warp for 16-byte words) on different banks.
+template <class H>
+struct SplitHalf : H {
+  static constexpr int E1S = H::R1 | 1;
+  static constexpr int WORDS = H::R0 * E1S;
+};
+template <class P>
+struct SplitCfg {
+  using H = typename P::H;
+  static constexpr int pad(int s, int r, int m) {
+    while (s % m != r) ++s;
+    return s;
+  }
+  static constexpr int w1 = SplitHalf<H>::WORDS, w2 = SplitHalf<typename Reverse<H>::type>::WORDS;
+  static constexpr int NEED = w1 > w2 ? w1 : w2;
+  static constexpr int OFF = pad(NEED, H::G < 8 ? H::G : 8, 16);   // 8-byte words
+  static constexpr int ROW = pad(2 * OFF, H::G < 8 ? 8 : 0, 16);
+  static constexpr int OFFP = pad(NEED, 4, 8);                     // 16-byte words
+};
+
 __device__ __forceinline__ float2 ldtw(const float2* __restrict__ tw, int j) { return __ldg(tw + j); }
 
 // 16-byte asynchronous global -> shared copy (L2 only) and its group fences.
@@ -348,6 +403,15 @@ template <class P>
 struct PlanTw {
   static constexpr int T2 = P::R0 * P::R1;
   static constexpr int SIZE = T2 + (P::R2 > 1 ? P::N : 0);
+};
+
+// Split2: the half plan's table, then the joining twiddles W_N^(point) of odd lanes (1 on even ones) in
+// register and lane order, for use as an inverse (output order) and as a forward (input order).
+template <class H>
+struct PlanTw<Split2<H>> {
+  static constexpr int T2 = PlanTw<H>::T2;
+  static constexpr int JOIN = PlanTw<H>::SIZE, VG = H::V * 2 * H::G;
+  static constexpr int SIZE = JOIN + 2 * VG;
 };
 
 // Executes stages of plan P on NT independent transforms held as v[t][V] by this thread.
@@ -425,6 +489,39 @@ __device__ __forceinline__ void fft_run(float2 (&v)[NT][P::V], float2* buf, int 
       }
 #pragma unroll
     for (int t = 0; t < NT; ++t) dft_groups<R2, DIR, true>(v[t]);
+  }
+}
+
+// One transform of a row held as v[V], exchanging through buf: fft_run, or the two halves and the step
+// that joins them.
+template <class P, int DIR, bool PK1, class SyncF>
+__device__ __forceinline__ void row_run(float2 (&v)[P::V], float2* buf, int g, const float2* __restrict__ tw, SyncF SYNC) {
+  if constexpr (IsSplit<P>::value) {
+    using H = SplitHalf<typename P::H>;
+    const int h = g & 1;
+    const float s = h ? -1.f : 1.f;
+    const float2 ss = make_float2(s, s);
+    const float2* jt = tw + PlanTw<P>::JOIN + (DIR > 0 ? 0 : PlanTw<P>::VG) + g;
+    if constexpr (DIR > 0) {
+      fft_run<H, DIR, 1, 0, 1, PK1>(reinterpret_cast<float2(&)[1][P::V]>(v), buf + h * SplitCfg<P>::OFF, 0, g >> 1, tw, SYNC);
+#pragma unroll
+      for (int i = 0; i < P::V; ++i) {  // X[k], X[k + N/2] = E +- W^k O
+        const float2 w = __ldg(jt + i * P::G);
+        const float2 t = cmul_cs<DIR>(v[i], w.x, w.y);
+        const float2 r = make_float2(__shfl_xor_sync(0xffffffffu, t.x, 1), __shfl_xor_sync(0xffffffffu, t.y, 1));
+        v[i] = paxpy(t, ss, r);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < P::V; ++i) {  // even outputs from x[n] + x[n + N/2], odd ones from (x[n] - x[n + N/2]) W^n
+        const float2 w = __ldg(jt + i * P::G);
+        const float2 r = make_float2(__shfl_xor_sync(0xffffffffu, v[i].x, 1), __shfl_xor_sync(0xffffffffu, v[i].y, 1));
+        v[i] = cmul_cs<DIR>(paxpy(v[i], ss, r), w.x, w.y);
+      }
+      fft_run<H, DIR, 1, 0, 1, PK1>(reinterpret_cast<float2(&)[1][P::V]>(v), buf + h * SplitCfg<P>::OFF, 0, g >> 1, tw, SYNC);
+    }
+  } else {
+    fft_run<P, DIR, 1, 0, 1, PK1>(reinterpret_cast<float2(&)[1][P::V]>(v), buf, 0, g, tw, SYNC);
   }
 }
 

@@ -142,6 +142,16 @@ struct PairRow {
   static constexpr int WORDS = S1 > S2 ? S1 : S2;
 };
 
+template <class H>
+struct PairRow<Split2<H>> {
+  static constexpr int WORDS = 2 * SplitCfg<Split2<H>>::OFFP;
+};
+// exchange strides of a half of a Split2
+template <class H>
+struct PairRow<SplitHalf<H>> {
+  static constexpr int E1S = SplitHalf<H>::E1S, E2S = 0, WORDS = SplitHalf<H>::WORDS;
+};
+
 // fft_run of two transforms held as v[V], exchanging through buf (PairRow<P>::WORDS 16-byte words).
 template <class P, int DIR, class SyncF>
 __device__ __forceinline__ void fft_run_pair(C2 (&v)[P::V], float4* buf, int g, const float2* __restrict__ tw, SyncF SYNC) {
@@ -189,6 +199,37 @@ __device__ __forceinline__ void fft_run_pair(C2 (&v)[P::V], float4* buf, int g, 
 #pragma unroll
       for (int n2 = 0; n2 < R2; ++n2) v[d * R2 + n2] = get(n2 * X::E2S + g + G * d);
     dft2_groups<R2, DIR>(v);
+  }
+}
+
+// row_run of two transforms.
+template <class P, int DIR, class SyncF>
+__device__ __forceinline__ void row_run_pair(C2 (&v)[P::V], float4* buf, int g, const float2* __restrict__ tw, SyncF SYNC) {
+  if constexpr (IsSplit<P>::value) {
+    using H = SplitHalf<typename P::H>;
+    const int h = g & 1;
+    const float s = h ? -1.f : 1.f;
+    const float2 ss = make_float2(s, s);
+    const float2* jt = tw + PlanTw<P>::JOIN + (DIR > 0 ? 0 : PlanTw<P>::VG) + g;
+    auto other = [](float2 a) { return make_float2(__shfl_xor_sync(0xffffffffu, a.x, 1), __shfl_xor_sync(0xffffffffu, a.y, 1)); };
+    if constexpr (DIR > 0) {
+      fft_run_pair<H, DIR>(v, buf + h * SplitCfg<P>::OFFP, g >> 1, tw, SYNC);
+#pragma unroll
+      for (int i = 0; i < P::V; ++i) {
+        const float2 w = __ldg(jt + i * P::G);
+        const C2 t = c2mul<DIR>(v[i], w.x, w.y);
+        v[i] = C2{paxpy(t.re, ss, other(t.re)), paxpy(t.im, ss, other(t.im))};
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < P::V; ++i) {
+        const float2 w = __ldg(jt + i * P::G);
+        v[i] = c2mul<DIR>(C2{paxpy(v[i].re, ss, other(v[i].re)), paxpy(v[i].im, ss, other(v[i].im))}, w.x, w.y);
+      }
+      fft_run_pair<H, DIR>(v, buf + h * SplitCfg<P>::OFFP, g >> 1, tw, SYNC);
+    }
+  } else {
+    fft_run_pair<P, DIR>(v, buf, g, tw, SYNC);
   }
 }
 

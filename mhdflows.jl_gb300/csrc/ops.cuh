@@ -170,6 +170,18 @@ class OpsBase {
 // precision rounded to FP32.
 template <class P>
 void plan_twiddles(std::vector<float2>& out) {
+  if constexpr (IsSplit<P>::value) {
+    using H = typename P::H;
+    plan_twiddles<H>(out);
+    for (int use = 0; use < 2; ++use)  // as an inverse: output order; as a forward: input order
+      for (int i = 0; i < P::V; ++i)
+        for (int g = 0; g < P::G; ++g) {
+          const int r = use ? P::R0 : P::RF, l = use ? H::LI : H::LF;
+          const double ang = 2.0 * 3.14159265358979323846 * (double)(g / 2 + H::G * (i / r) + l * (i % r)) / (double)P::N;
+          out.push_back(g % 2 ? make_float2((float)std::cos(ang), (float)std::sin(ang)) : make_float2(1.f, 0.f));
+        }
+    return;
+  }
   constexpr int N = P::N, R0 = P::R0, R1 = P::R1, R2 = P::R2;
   out.assign(PlanTw<P>::SIZE, make_float2(1.f, 0.f));
   auto w = [](long long j) {
@@ -186,6 +198,7 @@ void plan_twiddles(std::vector<float2>& out) {
 
 template <class P>
 std::string plan_name() {
+  if constexpr (IsSplit<P>::value) return "2x" + plan_name<typename P::H>();
   std::string s = std::to_string(P::R0) + "x" + std::to_string(P::R1);
   if (P::R2 > 1) s += "x" + std::to_string(P::R2);
   return s + "/g" + std::to_string(P::G);

@@ -74,13 +74,13 @@ OpsBase* make_ops_96() {
   auto* o = new Ops<96>();
   o->add_plane<Plan<96, 4, 8, 12>, 256, 2>();    // inverse 14.4, 66; forward 16.2, 68
   o->add_plane<Plan<96, 4, 8, 12>, 384, 2>(0);   // inverse 14.9, 64; forward 16.3, 72
-  o->add_x_tile<R, 2, 2>();
-  o->add_x_tile<R, 1, 2>();
+  using S = Split2<Plan<48, 4, 12, 4>>;
+  o->add_x_tile<S, 2, 2, 0, false, true>();      // 16.4, 83 (three-stage plan 16.5, 93; one buffer 17.2, 106)
   o->add_x_form<R, 1, 1, 1, 8, true, true>();
-  o->add_x_tile<R, 1, 2, 1>();
-  o->add_x_tile<R, 1, 2, 2>();
+  o->add_x_tile<S, 1, 2, 1>();                   // 22.7 (three-stage plan 24.6; two buffers leave one block per SM: 32.9)
+  o->add_x_tile<S, 1, 2, 2>();                   // with walls 26.7 (27.5)
   o->add_x_vp<R, 1, 1, 8, true>();
-  o->add_x_tile<R, 2, 2, 0, true>();
+  o->add_x_tile<S, 2, 2, 0, true, true>();       // hydrodynamics 13.2 (three-stage plan 14.4)
   o->add_x_hd<R, 1, 8, 0, true>();
   o->add_x_tile<R, 1, 2, 1, true>();
   o->add_x_tile<R, 1, 2, 2, true>();

@@ -647,7 +647,7 @@ struct RowCfg {
 template <class P, int VPM, bool HDX>
 __device__ __forceinline__ void x_pair(float2 (&w)[P::V], int t, const float2 (&v)[3][P::V], const float* chi,
                                        const float* __restrict__ wrow, long long cs, int g) {
-  constexpr int G = P::G, V = P::V, N = P::N;
+  constexpr int V = P::V, N = P::N;
 #pragma unroll
   for (int i = 0; i < V; ++i) {
     const float ux = v[0][i].x, uy = v[0][i].y, uz = v[1][i].x;
@@ -655,7 +655,7 @@ __device__ __forceinline__ void x_pair(float2 (&w)[P::V], int t, const float2 (&
     if (HDX && VPM > 0 && t >= 2) {
       if constexpr (HDX && VPM > 0) {
         constexpr float n3 = (float)N * (float)N * (float)N;
-        const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
+        const int x = phys_x<P>(g, i);
         auto wall = [&](int c) { return VPM == 2 ? n3 * __ldg(wrow + c * cs + x) : 0.f; };
         // scaled by n^3 to the products' magnitude (n^6 times physical): a pair whose halves
         // differ by n^3 would lose the small half to the large one's rounding in the split
@@ -668,7 +668,7 @@ __device__ __forceinline__ void x_pair(float2 (&w)[P::V], int t, const float2 (&
         float2 f = v[t - 4][i];
         if constexpr (VPM == 2) {  // the fields are n^3 times physical: so are the walls
           constexpr float n3 = (float)N * (float)N * (float)N;
-          const int x = g + G * (i / P::RF) + P::LF * (i % P::RF);
+          const int x = phys_x<P>(g, i);
           const long long c0 = (long long)(2 * (t - 4)) * cs;
           f.x = fmaf(-n3, __ldg(wrow + c0 + x), f.x);
           f.y = fmaf(-n3, __ldg(wrow + c0 + cs + x), f.y);
@@ -709,6 +709,11 @@ __device__ __forceinline__ void x_vmax(const float2 (&v)[3][V], unsigned int* vm
     atomicMax(vm + 1, bb);
   }
 }
+
+template <class H>
+struct RowCfg<Split2<H>> {
+  static constexpr int TS = SplitCfg<Split2<H>>::ROW;
+};
 
 // Fused x pass: per physical row (z, y): 3 inverse c2r pairs -> 6 physical fields -> 8 products
 // -> 4 forward r2c pairs -> 8 half-spectrum rows, written back over the same row slots.
@@ -756,6 +761,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
   using PR = typename Reverse<P>::type;
   constexpr int NTS = NTI > NTF ? NTI : NTF;
   using XC = XCfg<P, NTS, DIRECT, PAIR>;
+  static_assert(!IsSplit<P>::value || (NTI == 1 && NTF == 1 && P::G <= 32), "split rows go one at a time or in pairs");
   static_assert(!PAIR || (NTI == 1 && NTF == 1 && P::G <= 32), "pairs need the row inside one warp");
   static_assert(NTI == 1 || NTI == 3, "inverse transforms go one or three at a time");
   static_assert(NTF == 1 || NTF == 2 || NTF == 4, "forward transforms go one, two or four at a time");
@@ -845,7 +851,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       C2 z[V];
 #pragma unroll
       for (int i = 0; i < V; ++i) z[i] = C2{make_float2(v[0][i].x, v[1][i].x), make_float2(v[0][i].y, v[1][i].y)};
-      fft_run_pair<P, +1>(z, reinterpret_cast<float4*>(sb), g, tw, sync);
+      row_run_pair<P, +1>(z, reinterpret_cast<float4*>(sb), g, tw, sync);
       sync();
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -853,7 +859,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
         v[1][i] = make_float2(z[i].re.y, z[i].im.y);
       }
       if constexpr (!HDX) {
-        fft_run<P, +1, 1, TS, 1, false>(reinterpret_cast<float2(&)[1][V]>(v[2]), sb, 0, g, tw, sync);
+        row_run<P, +1, false>(v[2], sb, g, tw, sync);
         sync();
       }
     } else if constexpr (NTI == 3) {
@@ -862,7 +868,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
     } else {
 #pragma unroll
       for (int t = 0; t < NINV; ++t) {
-        fft_run<P, +1, 1, TS, 1, false>(reinterpret_cast<float2(&)[1][V]>(v[t]), sb, 0, g, tw, sync);
+        row_run<P, +1, false>(v[t], sb, g, tw, sync);
         sync();
       }
     }
@@ -890,9 +896,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       const float* crow = vp.chi + s * vp.cs + r * N;
       if constexpr (VPM == 2) wrow = vp.wall + 6 * s * vp.cs + r * N;
 #pragma unroll
-      for (int d = 0; d < P::DF; ++d)
-#pragma unroll
-        for (int e = 0; e < P::RF; ++e) chi[d * P::RF + e] = __ldg(crow + g + G * d + P::LF * e);
+      for (int i = 0; i < V; ++i) chi[i] = __ldg(crow + phys_x<P>(g, i));
     }
     // NTF product pairs at a time: the six fields stay live, each pair is formed just before its
     // forward transform (fewer live registers than all eight products at once)
@@ -913,7 +917,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
           C2 z[V];
 #pragma unroll
           for (int i = 0; i < V; ++i) z[i] = C2{make_float2(w[0][i].x, w[1][i].x), make_float2(w[0][i].y, w[1][i].y)};
-          fft_run_pair<PR, -1>(z, reinterpret_cast<float4*>(sb), g, twr, sync);
+          row_run_pair<PR, -1>(z, reinterpret_cast<float4*>(sb), g, twr, sync);
 #pragma unroll
           for (int i = 0; i < V; ++i) {
             w[0][i] = make_float2(z[i].re.x, z[i].im.x);
@@ -922,7 +926,7 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
           put_rows(w[0], t0);
           put_rows(w[1], t0 + 1);
         } else {
-          fft_run<PR, -1, 1, TS, 1>(reinterpret_cast<float2(&)[1][V]>(w[0]), sb, 0, g, twr, sync);
+          row_run<PR, -1, true>(w[0], sb, g, twr, sync);
           put_rows(w[0], t0);
         }
         sync();  // the next transform's first exchange overwrites sb
@@ -933,7 +937,8 @@ __global__ void __launch_bounds__(GROUPS * XCfg<P>::TPG, MINB)
       float2 w[NTF][V];
 #pragma unroll
       for (int j = 0; j < NTF; ++j) x_pair<P, VPM, HDX>(w[j], t0 + j, v, chi, wrow, vp.cs, g);
-      fft_run<PR, -1, NTF, TS, 1>(w, sb, 0, g, twr, sync);
+      if constexpr (NTF == 1) row_run<PR, -1, true>(w[0], sb, g, twr, sync);
+      else fft_run<PR, -1, NTF, TS, 1>(w, sb, 0, g, twr, sync);
       if constexpr (G <= 32) {
 #pragma unroll
         for (int j = 0; j < NTF; ++j)

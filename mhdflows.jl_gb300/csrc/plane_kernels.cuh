@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
       C2 c[V];
 #pragma unroll
       for (int i = 0; i < V; ++i) c[i] = C2{make_float2(v[0][i].x, v[1][i].x), make_float2(v[0][i].y, v[1][i].y)};
-      fft_run_pair<P, +1>(c, reinterpret_cast<float4*>(sb), g, tw, sync);
+      row_run_pair<P, +1>(c, reinterpret_cast<float4*>(sb), g, tw, sync);
       sync();
 #pragma unroll
       for (int i = 0; i < V; ++i) {
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
     }
 #pragma unroll
     for (int p = PAIR ? 2 : 0; p < NINV; ++p) {
-      fft_run<P, +1, 1, TS, 1, false>(reinterpret_cast<float2(&)[1][V]>(v[p]), sb, 0, g, tw, sync);
+      row_run<P, +1, false>(v[p], sb, g, tw, sync);
       sync();
     }
     if constexpr (HDX) {  // B = 0: the second half of pair 1 is zero up to roundoff, pair 2 unused
@@ -520,9 +520,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
       const float* crow = vp.chi + slot * vp.cs + row * N;
       if constexpr (VPM == 2) wrow = vp.wall + 6 * slot * vp.cs + row * N;
 #pragma unroll
-      for (int d = 0; d < P::DF; ++d)
-#pragma unroll
-        for (int e = 0; e < P::RF; ++e) chi[d * P::RF + e] = __ldg(crow + g + G * d + P::LF * e);
+      for (int i = 0; i < V; ++i) chi[i] = __ldg(crow + phys_x<P>(g, i));
     }
     // outputs over the row's own elements: its inputs are in registers, other rows' are elsewhere
     auto put_rows = [&](const float2(&w)[V], int p) {
@@ -540,7 +538,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
         C2 c[V];
 #pragma unroll
         for (int i = 0; i < V; ++i) c[i] = C2{make_float2(w[0][i].x, w[1][i].x), make_float2(w[0][i].y, w[1][i].y)};
-        fft_run_pair<PR, -1>(c, reinterpret_cast<float4*>(sb), g, twr, sync);
+        row_run_pair<PR, -1>(c, reinterpret_cast<float4*>(sb), g, twr, sync);
 #pragma unroll
         for (int i = 0; i < V; ++i) {
           w[0][i] = make_float2(c[i].re.x, c[i].im.x);
@@ -549,7 +547,7 @@ __global__ void __launch_bounds__(16 * P::G, MINB)
         put_rows(w[0], p);
         put_rows(w[1], p + 1);
       } else {
-        fft_run<PR, -1, 1, TS, 1>(reinterpret_cast<float2(&)[1][V]>(w[0]), sb, 0, g, twr, sync);
+        row_run<PR, -1, true>(w[0], sb, g, twr, sync);
         put_rows(w[0], p);
       }
       sync();  // the next transform's first exchange overwrites sb
