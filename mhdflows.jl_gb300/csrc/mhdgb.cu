@@ -398,6 +398,7 @@ struct mhd_problem {
   std::vector<long long> hist_step;
   std::vector<std::vector<double>> hist_t;
   cudaGraphExec_t graph_diag = nullptr;
+  cudaGraphExec_t graph_parked = nullptr, graph_diag_parked = nullptr;  // of the other divcorr setting
   // profiling
   bool profiling = false;
   bool tuning = false;  // a right-hand side also runs the fused inverse pass of its (unchanged) state
@@ -411,12 +412,11 @@ struct mhd_problem {
 
   void release() {
     cudaSetDevice(device);
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    if (graph_diag) cudaGraphExecDestroy(graph_diag);
-    graph_diag = nullptr;
-    if (graph_chain) cudaGraphExecDestroy(graph_chain);
-    graph_chain = nullptr;
+    drop(graph);
+    drop(graph_diag);
+    drop(graph_chain);
+    drop(graph_parked);
+    drop(graph_diag_parked);
     free_history();
     for (auto& r : recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     recs.clear();
@@ -830,14 +830,28 @@ struct mhd_problem {
       stepc[s] += 1;
     }
   }
+  static void drop(cudaGraphExec_t& g) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
   void invalidate_graph() {
-    if (graph) cudaGraphExecDestroy(graph);
-    graph = nullptr;
-    if (graph_diag) cudaGraphExecDestroy(graph_diag);
-    graph_diag = nullptr;
-    if (graph_chain) cudaGraphExecDestroy(graph_chain);
-    graph_chain = nullptr;
+    drop(graph);
+    drop(graph_diag);
+    drop(graph_chain);
+    drop(graph_parked);
+    drop(graph_diag_parked);
     graph_steps = 0;
+    ++graph_version;
+  }
+  // Switches the divergence corrections of a step.  TimeIntegrator does so around every run, so the
+  // step's graphs of the other setting are parked, not rebuilt (ten penalised steps at 128^3 with a
+  // capture and an instantiation 4.33 ms, without 4.21); a CFL step with corrections names the
+  // active slots in its launches and is captured anew.
+  void set_divcorr(bool on) {
+    if (cfl) invalidate_graph();
+    divcorr = on;
+    std::swap(graph, graph_parked);
+    std::swap(graph_diag, graph_diag_parked);
     ++graph_version;
   }
   int run_steps(int nsteps) {
@@ -1739,8 +1753,7 @@ int mhd_set_div_correction(mhd_handle h, int on) {
   if (on != 0 && on != 1) return fail(MHD_ERR_INVALID, "on must be 0 or 1");
   if ((on != 0) != h->divcorr) {
     MHD_CUDA(cudaStreamSynchronize(h->stream));
-    h->divcorr = on != 0;
-    h->invalidate_graph();
+    h->set_divcorr(on != 0);
   }
   return MHD_OK;
 }
@@ -1751,21 +1764,30 @@ int mhd_set_diag_history(mhd_handle h, int freq, int capacity) {
   if (freq < 0 || capacity < 0 || (freq > 0 && capacity < 1))
     return fail(MHD_ERR_INVALID, "freq >= 0 and, with freq > 0, capacity >= 1 required");
   MHD_CUDA(cudaStreamSynchronize(h->stream));
-  h->free_history();
+  // the same capacity again keeps the buffers and the recording step's graph, which names them
+  const int cap_new = freq > 0 ? capacity : 0;
+  const bool keep = h->dhist && cap_new == h->diag_capacity;
   h->hist_step.clear();
   h->hist_t.clear();
   h->hsteps = 0;
-  h->diag_freq = freq;
-  h->diag_capacity = freq > 0 ? capacity : 0;
+  h->diag_freq = h->diag_capacity = 0;  // off until the buffers are there
+  if (!keep) {
+    h->free_history();
+    h->drop(h->graph_diag);
+    h->drop(h->graph_diag_parked);
+    if (freq > 0) {
+      const size_t c = (size_t)h->cap;
+      MHD_CUDA(cudaMalloc(&h->dhist, (size_t)capacity * c * kHistVals * sizeof(double)));
+      MHD_CUDA(cudaMalloc(&h->dhist_partial, c * h->sz.diag_blocks * kDiagSlots * sizeof(double)));
+      MHD_CUDA(cudaMalloc(&h->dhist_count, sizeof(int)));
+    }
+  }
   if (freq > 0) {
-    const size_t c = (size_t)h->cap;
-    MHD_CUDA(cudaMalloc(&h->dhist, (size_t)capacity * c * kHistVals * sizeof(double)));
-    MHD_CUDA(cudaMalloc(&h->dhist_partial, c * h->sz.diag_blocks * kDiagSlots * sizeof(double)));
-    MHD_CUDA(cudaMalloc(&h->dhist_count, sizeof(int)));
     MHD_CUDA(cudaMemsetAsync(h->dhist_count, 0, sizeof(int), h->stream));
     MHD_CUDA(cudaStreamSynchronize(h->stream));
   }
-  h->invalidate_graph();
+  h->diag_freq = freq;
+  h->diag_capacity = cap_new;
   return MHD_OK;
 }
 
@@ -1846,6 +1868,9 @@ int mhd_set_cfl(mhd_handle h, int enable, double coef) {
   if (enable && !(coef > 0 && std::isfinite(coef))) return fail(MHD_ERR_INVALID, "CFL coefficient must be positive");
   if ((rc = h->sync_lists())) return rc;
   MHD_CUDA(cudaStreamSynchronize(h->stream));
+  // the step's launches depend on the switch and on the coefficient alone (with the corrections also on
+  // the active slots): a repeated call keeps its graphs
+  if ((enable != 0) != h->cfl || (enable && (coef != h->cfl_coef || h->divcorr))) h->invalidate_graph();
   if (enable) {
     h->cfl_coef = coef;
     const double dl = h->p.L / h->g.n;
@@ -1857,8 +1882,11 @@ int mhd_set_cfl(mhd_handle h, int enable, double coef) {
     if ((rc = h->sync_lists())) return rc;
     MHD_CUDA(cudaMemcpyAsync(h->dtime, h->t.data(), h->cap * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     h->cfl = true;
-    if ((rc = h->cfl_prime())) { h->cfl = false; return rc; }
-    if ((rc = h->cfl_update(0))) { h->cfl = false; return rc; }
+    if ((rc = h->cfl_prime()) || (rc = h->cfl_update(0))) {
+      h->cfl = false;
+      h->invalidate_graph();
+      return rc;
+    }
     std::vector<SlotParams> dev(h->cap);
     MHD_CUDA(cudaMemcpyAsync(dev.data(), h->dparams, h->cap * sizeof(SlotParams), cudaMemcpyDeviceToHost, h->stream));
     MHD_CUDA(cudaStreamSynchronize(h->stream));
@@ -1871,7 +1899,6 @@ int mhd_set_cfl(mhd_handle h, int enable, double coef) {
     for (int s = 0; s < h->cap; ++s) h->hparams[s].dt = dev[s].dt;
     h->cfl = false;
   }
-  h->invalidate_graph();
   return MHD_OK;
 }
 

@@ -84,3 +84,27 @@ def test_chained_steps_equal_single_ones(pkg, mo, n, scheme, cfl):
             got.append((prob.sol_c(), prob.clock.t, prob.clock.step))
     assert np.array_equal(got[0][0], got[1][0])
     assert got[0][1:] == got[1][1:]
+
+
+@pytest.mark.parametrize("form,cfl", [("mhd", True), ("mhdvp", False), ("mhdvp", True)])
+def test_runs_on_kept_graphs_equal_runs_on_new_ones(pkg, mo, form, cfl):
+    """Runs after one another keep the step's graphs: states, clocks and recorded diagnostics agree bit
+    for bit with those of a handle whose graphs are dropped before every run (by selecting the
+    variant it has)."""
+    got = []
+    for fresh in (False, True):
+        _, _, prob, _ = _problem(pkg, mo, 32, form, dt=1e-4)
+        with prob:
+            out = []
+            names = pkg.variants(prob)["x_fused"]
+            for steps, freq in ((3, 2), (4, 0), (3, 2), (5, 1), (3, 1)):
+                if fresh:
+                    pkg.select_variant(prob, "x_fused", names[1].index(names[0]))
+                pkg.TimeIntegrator(prob, math.inf, steps - 1, usr_dt=0.0 if cfl else 1e-4, diag_freq=freq)
+                if freq:
+                    out.append(prob.diagnostic_history())
+                pkg.stepforward(prob, 2)
+                out += [prob.sol_c(), np.array([prob.clock.t, prob.clock.dt])]
+            got.append(out)
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
