@@ -58,15 +58,23 @@ __device__ __forceinline__ float a99_uniform(unsigned long long key, unsigned lo
   return (float)(z >> 40) * (1.0f / 16777216.0f);
 }
 // forcing of the three velocity components at wavenumber (kx, ky, kz)
+// A mode whose Gaussian underflows to zero (at sigma = 1 every mode more than 10.2 from the peak: all but
+// 1 % of the band at 128^3) gets exactly zero, whatever is drawn: it skips the draws and the functions
+// of them (a stage at 128^3 43 -> 17 us in a low-storage run, where the unforced one takes 15).
 __device__ __forceinline__ void a99_force(const SlotParams& sp, unsigned long long key, unsigned long long index,
                                           float kx, float ky, float kz, float2 (&F)[3]) {
   constexpr float kPi = 3.14159265358979f;
   const float k = sqrtf(kx * kx + ky * ky + kz * kz);
+  const float dk = k - sp.fkf;
+  const float gauss = expf(-dk * dk / sp.fs2);
+  if (gauss == 0.f && isfinite(sp.fA) && sp.fb != 0.f) {  // fb = 0 and an infinite fA give NaN at every mode
+    F[0] = F[1] = F[2] = make_float2(0.f, 0.f);
+    return;
+  }
   const float kp = sqrtf(kx * kx + kz * kz);
   const float kinv = k > 0.f ? 1.f / k : 0.f;
   const float pinv = kp > 0.f ? 1.f / kp : 0.f;
-  const float dk = k - sp.fkf;
-  const float Fk = sp.fA * sqrtf(expf(-dk * dk / sp.fs2) / 2.f / kPi) * kinv;
+  const float Fk = sp.fA * sqrtf(gauss / 2.f / kPi) * kinv;
   const float e1x = kz * pinv, e1z = -kx * pinv;
   const float e2x = kx * ky * pinv * kinv, e2y = -kp * kinv, e2z = kz * ky * pinv * kinv;
   const float th1 = a99_uniform(key, index, 0) * 2.f * kPi;
