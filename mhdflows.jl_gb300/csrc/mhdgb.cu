@@ -131,7 +131,7 @@ Sizes sizes_of(const Geom& g, int ns) {
   s.ref = 6LL * (g.n / 2 + 1) * g.n * g.n;
   s.phys = (long long)g.n * g.n * g.n;
   long long b = (s.fs + kDiagThreads - 1) / kDiagThreads;
-  s.diag_blocks = (int)(b < 1216 ? b : 1216);
+  s.diag_blocks = (int)(b < kDiagBlocks ? b : kDiagBlocks);
   return s;
 }
 
@@ -310,7 +310,6 @@ struct mhd_problem {
   float* phys = nullptr;
   double* diag_partial = nullptr;
   double* diag_out = nullptr;
-  unsigned int* maxabs = nullptr;
   // work lists
   SlotParams* dparams = nullptr;
   int* dlist = nullptr;
@@ -431,13 +430,13 @@ struct mhd_problem {
     zstream = nullptr;
     zeros = nullptr;
     ev_z = nullptr;
-    void* ptrs[] = {sol, xs, acc, aux, colbuf, rowbuf, ref, phys, diag_partial, diag_out, maxabs, dparams, dlist, dvmax, dtime,
+    void* ptrs[] = {sol, xs, acc, aux, colbuf, rowbuf, ref, phys, diag_partial, diag_out, dparams, dlist, dvmax, dtime,
                     dstep, derr, vchi, vwall};
     for (void* q : ptrs) if (q) cudaFree(q);
     vchi = vwall = nullptr;
     sol = xs = acc = aux = colbuf = rowbuf = ref = nullptr;
     guards.clear();
-    phys = nullptr; diag_partial = nullptr; diag_out = nullptr; maxabs = nullptr; dparams = nullptr; dlist = nullptr;
+    phys = nullptr; diag_partial = nullptr; diag_out = nullptr; dparams = nullptr; dlist = nullptr;
     dvmax = nullptr; dtime = nullptr; dstep = nullptr; derr = nullptr;
     if (own_stream) cudaStreamDestroy(own_stream);
     own_stream = nullptr;
@@ -700,6 +699,13 @@ struct mhd_problem {
                                                               advance);
     });
   }
+  // max |x| of the physical staging array into *out (its size is a multiple of 16)
+  int maxabs(unsigned int* out) {
+    const long long n4 = sz.phys / 4, blocks = std::min<long long>((n4 + kDiagThreads - 1) / kDiagThreads, 1216);
+    return launch(KC_OTHER, [&] {
+      maxabs_kernel<<<(unsigned)blocks, kDiagThreads, 0, stream>>>(reinterpret_cast<const float4*>(phys), n4, out);
+    });
+  }
   // maxima of the current state's physical fields (the first CFL step's vars)
   int cfl_prime() {
     int rc;
@@ -708,7 +714,7 @@ struct mhd_problem {
       for (int f = 0; f < 6; ++f) {
         if ((rc = inverse_field(sol + f * sz.fs, sz.state, s, 1.0f))) return rc;  // raw units, like x_fused
         unsigned int* out = dvmax + 2 * s + (f < 3 ? 0 : 1);
-        if ((rc = launch(KC_OTHER, [&] { maxabs_into_kernel<<<1216, 256, 0, stream>>>(phys, sz.phys, out); }))) return rc;
+        if ((rc = maxabs(out))) return rc;
       }
     return MHD_OK;
   }
@@ -1064,7 +1070,6 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   MHD_CUDA(h->alloc_guarded(&h->phys, s.phys * sizeof(float)));
   MHD_CUDA(cudaMalloc(&h->diag_partial, (size_t)s.diag_blocks * kDiagSlots * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->diag_out, 16 * sizeof(double)));
-  MHD_CUDA(cudaMalloc(&h->maxabs, 16 * sizeof(unsigned int)));
   MHD_CUDA(cudaMalloc(&h->dparams, c * sizeof(SlotParams)));
   MHD_CUDA(cudaMalloc(&h->dlist, (2 * c + 2) * sizeof(int)));
   MHD_CUDA(cudaMalloc(&h->dvmax, 2 * c * sizeof(unsigned int)));
@@ -1909,22 +1914,19 @@ int mhd_slot_diagnostics(mhd_handle h, int slot, double* out, int nout) {
   const Sizes& s = h->sz;
   const float2* st = h->sol + slot * s.state;
   float2* aux = h->aux + slot * s.fs;
-  if ((rc = h->launch(KC_OTHER, [&] { diag_partial_kernel<<<s.diag_blocks, kDiagThreads, 0, h->stream>>>(st, h->g, h->diag_partial); }))) return rc;
+  if ((rc = h->launch(KC_OTHER, [&] { diag_partial_kernel<<<s.diag_blocks, kDiagThreads, 0, h->stream>>>(st, h->g, h->diag_partial, aux); }))) return rc;
   if ((rc = h->launch(KC_OTHER, [&] { diag_final_kernel<<<1, kDiagThreads, 0, h->stream>>>(h->diag_partial, s.diag_blocks, h->diag_out); }))) return rc;
-  if ((rc = h->launch(KC_OTHER, [&] { divb_spectrum_kernel<<<1216, 256, 0, h->stream>>>(st, aux, h->g); }))) return rc;
   if ((rc = h->inverse_field(h->aux, s.fs, slot))) return rc;
-  MHD_CUDA(cudaMemsetAsync(h->maxabs, 0, sizeof(unsigned int), h->stream));
-  if ((rc = h->launch(KC_OTHER, [&] { maxabs_kernel<<<1216, 256, 0, h->stream>>>(h->phys, s.phys, h->maxabs); }))) return rc;
-  double d[kDiagSlots];
-  unsigned int mx = 0;
+  unsigned int* maxabs = reinterpret_cast<unsigned int*>(h->diag_out + kDiagSlots);
+  if ((rc = h->maxabs(maxabs))) return rc;
+  double d[kDiagSlots + 1];
   MHD_CUDA(cudaMemcpyAsync(d, h->diag_out, sizeof(d), cudaMemcpyDeviceToHost, h->stream));
-  MHD_CUDA(cudaMemcpyAsync(&mx, h->maxabs, sizeof(mx), cudaMemcpyDeviceToHost, h->stream));
   MHD_CUDA(cudaStreamSynchronize(h->stream));
   const double n3 = (double)h->g.n * h->g.n * h->g.n;
   const double dx = h->p.L / h->g.n;
   const double scale = dx * dx * dx / n3;
   float mxf;
-  std::memcpy(&mxf, &mx, sizeof(mxf));
+  std::memcpy(&mxf, d + kDiagSlots, sizeof(mxf));
   out[0] = d[0] * scale;
   out[1] = d[1] * scale;
   out[2] = d[2] * scale;

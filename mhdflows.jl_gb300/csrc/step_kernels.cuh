@@ -113,16 +113,6 @@ __global__ void step_tick_kernel(BatchRef br, long long* steps) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) steps[br.slot(i)] += 1;
 }
 
-// max |field| of one physical field into vmax[which] (initial fields before the first CFL step).
-__global__ void maxabs_into_kernel(const float* __restrict__ a, long long n, unsigned int* out) {
-  unsigned int m = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    m = max(m, __float_as_uint(fabsf(a[i])));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 // ------------------------------------------------------------------------------------------
 // Layout conversion between the reference's column-major sol[kx, ky, kz, f] (half spectrum,
 // nkr = n/2+1) and the compact retained-band state.
@@ -197,6 +187,9 @@ __global__ void __launch_bounds__(kCopyThreads) scatter_retained_kernel(const fl
 // w = 1 on the kx = 0 plane and 2 elsewhere (the half spectrum stands for both +-kx).
 constexpr int kDiagSlots = 6;
 constexpr int kDiagThreads = 256;
+// Blocks per state: one per SM.  A block's reduction of FP64 sums costs as much of the FP64 pipe as half a mode per
+// thread, so few threads with many modes each (8 at 128^3) beat many threads with one.
+constexpr int kDiagBlocks = 152;
 
 __device__ __forceinline__ void block_reduce_diag(double (&acc)[kDiagSlots], double* out) {
   __shared__ double red[kDiagThreads / 32][kDiagSlots];
@@ -220,38 +213,65 @@ __device__ __forceinline__ void block_reduce_diag(double (&acc)[kDiagSlots], dou
   }
 }
 
-__global__ void __launch_bounds__(kDiagThreads) diag_partial_kernel(const float2* __restrict__ S, Geom geo, double* partial) {
-  const long long plane = field_elems(geo);
-  double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
-    int x, jy, jz;
-    if (!mode_at(geo, i, x, jy, jz)) continue;
+// One mode into a thread's sums.  The kernels that call this are bound by the FP64 pipe (2 FMA per clock and
+// SM): the maxima are taken of the squares and rooted once a thread (the rounded square root is monotone, so
+// the maximum is the same to the bit), which left 57 of about 100 FP64 instructions a mode.  Recorded
+// diagnostics with kDiagBlocks: 128^3 78 -> 49 us, 256^3 409 -> 315.
+struct DiagAcc {
+  double v[kDiagSlots] = {0, 0, 0, 0, 0, 0};
+  int bad = 0;
+  __device__ __forceinline__ void mode(const Geom& geo, const float2 (&u)[3], const float2 (&b)[3], int x, int jy, int jz) {
     const double w = x == 0 ? 1.0 : 2.0;
-    const double kx = (double)geo.kscale * x;
-    const double ky = (double)geo.kscale * signed_of_kept(geo, jy);
-    const double kz = (double)geo.kscale * signed_of_kept(geo, jz);
+    const double k[3] = {(double)geo.kscale * x, (double)geo.kscale * signed_of_kept(geo, jy), (double)geo.kscale * signed_of_kept(geo, jz)};
     double2 ku = make_double2(0, 0), kb = make_double2(0, 0);
     double eu = 0, eb = 0, hc = 0;
-    bool bad = false;
+    bool nf = false;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const float2 u = S[c * geo.fs + i], b = S[(c + 3) * geo.fs + i];
-      bad |= !isfinite(u.x) || !isfinite(u.y) || !isfinite(b.x) || !isfinite(b.y);
-      eu += (double)u.x * u.x + (double)u.y * u.y;
-      eb += (double)b.x * b.x + (double)b.y * b.y;
-      hc += (double)u.x * b.x + (double)u.y * b.y;
-      const double kc = c == 0 ? kx : (c == 1 ? ky : kz);
-      ku.x += kc * u.x; ku.y += kc * u.y;
-      kb.x += kc * b.x; kb.y += kc * b.y;
+      nf |= !isfinite(u[c].x) || !isfinite(u[c].y) || !isfinite(b[c].x) || !isfinite(b[c].y);
+      eu += (double)u[c].x * u[c].x + (double)u[c].y * u[c].y;
+      eb += (double)b[c].x * b[c].x + (double)b[c].y * b[c].y;
+      hc += (double)u[c].x * b[c].x + (double)u[c].y * b[c].y;
+      ku.x += k[c] * u[c].x; ku.y += k[c] * u[c].y;
+      kb.x += k[c] * b[c].x; kb.y += k[c] * b[c].y;
     }
-    acc[0] += w * eu;
-    acc[1] += w * eb;
-    acc[2] += w * hc;
-    acc[3] = fmax(acc[3], sqrt(ku.x * ku.x + ku.y * ku.y));
-    acc[4] = fmax(acc[4], sqrt(kb.x * kb.x + kb.y * kb.y));
-    acc[5] += bad ? 1.0 : 0.0;
+    v[0] += w * eu;
+    v[1] += w * eb;
+    v[2] += w * hc;
+    v[3] = fmax(v[3], ku.x * ku.x + ku.y * ku.y);
+    v[4] = fmax(v[4], kb.x * kb.x + kb.y * kb.y);
+    bad += nf;
   }
-  block_reduce_diag(acc, partial + (long long)blockIdx.x * kDiagSlots);
+  __device__ __forceinline__ void finish() {
+    v[3] = sqrt(v[3]);
+    v[4] = sqrt(v[4]);
+    v[5] = bad;
+  }
+};
+
+// Sums of one state, and i k.B as a one-field compact buffer (input of the div B inverse transform).
+__global__ void __launch_bounds__(kDiagThreads) diag_partial_kernel(const float2* __restrict__ S, Geom geo, double* partial,
+                                                                    float2* __restrict__ divb) {
+  const long long plane = field_elems(geo);
+  DiagAcc acc;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
+    int x, jy, jz;
+    if (!mode_at(geo, i, x, jy, jz)) {
+      divb[i] = make_float2(0.f, 0.f);
+      continue;
+    }
+    float2 u[3], b[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      u[c] = S[c * geo.fs + i];
+      b[c] = S[(c + 3) * geo.fs + i];
+    }
+    const float kx = geo.kscale * x, ky = geo.kscale * signed_of_kept(geo, jy), kz = geo.kscale * signed_of_kept(geo, jz);
+    divb[i] = make_float2(-(kx * b[0].y + ky * b[1].y + kz * b[2].y), kx * b[0].x + ky * b[1].x + kz * b[2].x);
+    acc.mode(geo, u, b, x, jy, jz);
+  }
+  acc.finish();
+  block_reduce_diag(acc.v, partial + (long long)blockIdx.x * kDiagSlots);
 }
 
 // Second pass: reduce the block partials in block order (deterministic).
@@ -265,6 +285,7 @@ __global__ void __launch_bounds__(kDiagThreads) diag_final_kernel(const double* 
     }
   }
   block_reduce_diag(acc, out);
+  if (threadIdx.x == 0) out[kDiagSlots] = 0.0;  // where max |div B| is gathered next (its bits, maxabs_kernel)
 }
 
 // On-device diagnostics history (getCFL! / increment!(diags) without host synchronisation):
@@ -277,36 +298,20 @@ __global__ void __launch_bounds__(kDiagThreads) diag_partial_batch_kernel(const 
   const int slot = br.slot(inst);
   const float2* S = pool + slot * stI;
   const long long plane = field_elems(geo);
-  double acc[kDiagSlots] = {0, 0, 0, 0, 0, 0};
+  DiagAcc acc;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
     int x, jy, jz;
     if (!mode_at(geo, i, x, jy, jz)) continue;
-    const double w = x == 0 ? 1.0 : 2.0;
-    const double kx = (double)geo.kscale * x;
-    const double ky = (double)geo.kscale * signed_of_kept(geo, jy);
-    const double kz = (double)geo.kscale * signed_of_kept(geo, jz);
-    double2 ku = make_double2(0, 0), kb = make_double2(0, 0);
-    double eu = 0, eb = 0, hc = 0;
-    bool bad = false;
+    float2 u[3], b[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const float2 u = S[c * geo.fs + i], b = S[(c + 3) * geo.fs + i];
-      bad |= !isfinite(u.x) || !isfinite(u.y) || !isfinite(b.x) || !isfinite(b.y);
-      eu += (double)u.x * u.x + (double)u.y * u.y;
-      eb += (double)b.x * b.x + (double)b.y * b.y;
-      hc += (double)u.x * b.x + (double)u.y * b.y;
-      const double kc = c == 0 ? kx : (c == 1 ? ky : kz);
-      ku.x += kc * u.x; ku.y += kc * u.y;
-      kb.x += kc * b.x; kb.y += kc * b.y;
+      u[c] = S[c * geo.fs + i];
+      b[c] = S[(c + 3) * geo.fs + i];
     }
-    acc[0] += w * eu;
-    acc[1] += w * eb;
-    acc[2] += w * hc;
-    acc[3] = fmax(acc[3], sqrt(ku.x * ku.x + ku.y * ku.y));
-    acc[4] = fmax(acc[4], sqrt(kb.x * kb.x + kb.y * kb.y));
-    acc[5] += bad ? 1.0 : 0.0;
+    acc.mode(geo, u, b, x, jy, jz);
   }
-  block_reduce_diag(acc, partial + ((long long)slot * gridDim.x + blockIdx.x) * kDiagSlots);
+  acc.finish();
+  block_reduce_diag(acc.v, partial + ((long long)slot * gridDim.x + blockIdx.x) * kDiagSlots);
 }
 
 // grid (cap): one block per instance reduces its slot's partials (block order, deterministic)
@@ -347,20 +352,6 @@ __global__ void __launch_bounds__(kDiagThreads) diag_record_kernel(const double*
 }
 __global__ void hist_tick_kernel(int* count) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *count += 1;
-}
-
-// i k.B into a one-field compact buffer (input of the div B inverse transform).
-__global__ void divb_spectrum_kernel(const float2* __restrict__ S, float2* __restrict__ out, Geom geo) {
-  const long long plane = field_elems(geo);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x) {
-    int x, jy, jz;
-    const bool in = mode_at(geo, i, x, jy, jz);
-    const float kx = geo.kscale * x, ky = geo.kscale * signed_of_kept(geo, jy), kz = geo.kscale * signed_of_kept(geo, jz);
-    const float2 bx = S[3 * geo.fs + i], by = S[4 * geo.fs + i], bz = S[5 * geo.fs + i];
-    const float re = kx * bx.x + ky * by.x + kz * bz.x;
-    const float im = kx * bx.y + ky * by.y + kz * bz.y;
-    out[i] = in ? make_float2(-im, re) : make_float2(0.f, 0.f);
-  }
 }
 
 // DivVCorrection! / DivBCorrection! (src/Solver/VPSolver.jl:60-138): u (mask bit 0) and B (bit 1)
@@ -415,19 +406,26 @@ __global__ void guard_check_kernel(const unsigned char* __restrict__ g, long lon
   if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(bad, (unsigned long long)cnt);
 }
 
-// max |x| over a float array via the ordered bit pattern of non-negative floats (NaN wins).
-__global__ void maxabs_kernel(const float* __restrict__ a, long long n, unsigned int* out) {
+// max |x| over a float array via the ordered bit pattern of non-negative floats (NaN wins), into *out, which
+// the caller has cleared.  One atomic a block: with one a warp they took longer than the reads up to 128^3.
+__global__ void __launch_bounds__(kDiagThreads) maxabs_kernel(const float4* __restrict__ a, long long n4, unsigned int* out) {
+  __shared__ unsigned int red[kDiagThreads / 32];
   unsigned int m = 0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const unsigned int b = __float_as_uint(fabsf(a[i]));
-    m = b > m ? b : m;
+  auto take = [&](float x) { m = max(m, __float_as_uint(fabsf(x))); };
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const float4 q = a[i];
+    take(q.x);
+    take(q.y);
+    take(q.z);
+    take(q.w);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned int y = __shfl_down_sync(0xffffffffu, m, o);
-    m = y > m ? y : m;
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = __reduce_max_sync(0xffffffffu, threadIdx.x < kDiagThreads / 32 ? red[threadIdx.x] : 0u);
+    if (threadIdx.x == 0) atomicMax(out, m);
   }
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
 }  // namespace mhdgb
