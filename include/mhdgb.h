@@ -104,6 +104,8 @@ int mhd_get_state_device(mhd_handle h, float* sol_dev, void* stream);
 
 /* SetUpProblemIC!: physical field (n, n, n) float32 column-major -> forward r2c into sol[:,:,:,field]. */
 int mhd_set_physical(mhd_handle h, int field, const float* phys);
+/* The same, and the array itself into copy (host, n^3 floats; it may be phys). */
+int mhd_set_physical_copy(mhd_handle h, int field, const float* phys, float* copy);
 /* updatevars!: vars.<field> <- normalised c2r of sol[:,:,:,field]. field 0..5 = ux uy uz bx by bz. */
 int mhd_get_physical(mhd_handle h, int field, float* phys);
 

@@ -381,6 +381,15 @@ def _to_c_phys(a, n):
     return np.ascontiguousarray(np.asarray(a, dtype=np.float32).T)
 
 
+def _vars_memory(prob, f):
+    """Address of the vars array of field f if the library can write it in place (float32 in
+    column-major order, as Vars lays it out), else None: an array of another kind was put there."""
+    a = getattr(prob.vars, FIELDS[f])
+    ok = (isinstance(a, np.ndarray) and a.dtype == np.float32 and a.shape == (prob.n,) * 3 and a.flags.f_contiguous
+          and a.flags.writeable and a.flags.aligned and a.dtype.isnative)
+    return a.ctypes.data if ok else None
+
+
 def SetUpProblemIC(prob: Problem, *, ux=None, uy=None, uz=None, bx=None, by=None, bz=None):
     """SetUpProblemIC!(prob; ux, ..., bz) (src/utils/IC.jl:41-109): host field -> device -> r2c."""
     for f, arr in enumerate((ux, uy, uz, bx, by, bz)):
@@ -389,8 +398,12 @@ def SetUpProblemIC(prob: Problem, *, ux=None, uy=None, uz=None, bx=None, by=None
         if f >= prob.nfields:
             raise MHDError(_lib.MHD_ERR_INVALID, "a hydrodynamic problem (B_field=false) has no magnetic field")
         c = _to_c_phys(arr, prob.n)
-        prob.set_physical_c(f, c)
-        getattr(prob.vars, FIELDS[f])[...] = c.T
+        v = _vars_memory(prob, f)
+        if v is None:
+            prob.set_physical_c(f, c)
+            getattr(prob.vars, FIELDS[f])[...] = c.T
+        else:
+            _lib.check(prob._lib.mhd_set_physical_copy(prob._h, f, c.ctypes.data, v))
     return None
 
 
@@ -413,7 +426,11 @@ def stepforward(prob: Problem, nsteps: int = 1):
 def updatevars(prob: Problem):
     """updatevars!(prob): vars.ux..bz <- normalised c2r of the current sol."""
     for f, name in enumerate(FIELDS[: prob.nfields]):
-        getattr(prob.vars, name)[...] = prob.physical_c(f).T
+        v = _vars_memory(prob, f)
+        if v is None:
+            getattr(prob.vars, name)[...] = prob.physical_c(f).T
+        else:
+            _lib.check(prob._lib.mhd_get_physical(prob._h, f, v))
     return None
 
 

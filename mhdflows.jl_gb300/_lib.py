@@ -87,6 +87,7 @@ _SIGS = {
     "mhd_set_state": (C.c_int, [C.c_void_p, C.c_void_p]),
     "mhd_get_state": (C.c_int, [C.c_void_p, C.c_void_p]),
     "mhd_set_physical": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p]),
+    "mhd_set_physical_copy": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "mhd_get_physical": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p]),
     "mhd_step": (C.c_int, [C.c_void_p, C.c_int]),
     "mhd_compute_rhs": (C.c_int, [C.c_void_p, C.c_void_p]),

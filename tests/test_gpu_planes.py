@@ -108,3 +108,27 @@ def test_runs_on_kept_graphs_equal_runs_on_new_ones(pkg, mo, form, cfl):
             got.append(out)
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("order,dtype", [("F", np.float32), ("C", np.float32), ("F", np.float64)])
+def test_vars_arrays_in_place_and_replaced(pkg, mo, order, dtype):
+    """SetUpProblemIC and updatevars fill the vars arrays in place where their memory is the library's
+    layout, and through a copy where the caller put another kind of array there: same values, and
+    the fields handed in stay as they were (also when they are the vars arrays)."""
+    n = 32
+    _, s, prob, _ = _problem(pkg, mo, n, "mhd")
+    rng = np.random.default_rng(0)
+    f = rng.standard_normal((n, n, n)).astype(np.float32)
+    with prob:
+        for name in ("ux", "bz"):
+            setattr(prob.vars, name, np.zeros((n, n, n), dtype=dtype, order=order))
+        keep = f.copy()
+        pkg.SetUpProblemIC(prob, ux=f, bz=np.asfortranarray(f))
+        assert np.array_equal(f, keep) and np.array_equal(prob.vars.ux, f) and np.array_equal(prob.vars.bz, f)
+        pkg.SetUpProblemIC(prob, ux=prob.vars.ux)
+        assert np.array_equal(prob.vars.ux, f)
+        arrays = [prob.vars.ux, prob.vars.by]
+        pkg.updatevars(prob)
+        assert prob.vars.ux is arrays[0] and prob.vars.by is arrays[1]
+        for i, name in enumerate(pkg.FIELDS):
+            assert np.array_equal(getattr(prob.vars, name), prob.physical_c(i).T)
