@@ -335,7 +335,7 @@ struct mhd_problem {
   int* derr = nullptr;
   bool cfl = false;
   double cfl_coef = 0.3;
-  int graph_version = 0;   // active slots, then the identity list (cap each), then counts
+  int graph_version = 0;   // counts the changes of what a step launches (ensembles re-capture)
   std::vector<SlotParams> hparams;
   std::vector<char> used;
   std::vector<int> active;
@@ -442,17 +442,20 @@ struct mhd_problem {
     own_stream = nullptr;
   }
 
-  // device work lists: dlist[0..cap) active, dlist[cap..2cap) identity, dlist[2cap] active count, dlist[2cap+1] = 1
-  BatchRef active_ref() const { return BatchRef{dlist, dlist + 2 * cap, cap == 1}; }
-  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 2 * cap + 1, cap == 1}; }
+  // device work lists: dlist[0..cap) active, dlist[cap..3cap) identity, dlist[3cap] active count, dlist[3cap+1] = 1.
+  // Every kernel may look up any instance below the capacity, active or not (the plane and stage kernels
+  // issue their first loads before they know the count): the entries past the active ones are
+  // slot 0, and slot_ref's list, which starts at the slot's own entry, runs on with the last slot.
+  BatchRef active_ref() const { return BatchRef{dlist, dlist + 3 * cap, cap == 1}; }
+  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 3 * cap + 1, cap == 1}; }
 
   int sync_lists() {
     if (!list_dirty) return MHD_OK;
-    std::vector<int> h(2 * cap + 2, 0);
+    std::vector<int> h(3 * cap + 2, 0);
     for (size_t i = 0; i < active.size(); ++i) h[i] = active[i];
-    for (int i = 0; i < cap; ++i) h[cap + i] = i;
-    h[2 * cap] = (int)active.size();
-    h[2 * cap + 1] = 1;
+    for (int i = 0; i < 2 * cap; ++i) h[cap + i] = std::min(i, cap - 1);
+    h[3 * cap] = (int)active.size();
+    h[3 * cap + 1] = 1;
     MHD_CUDA(cudaMemcpyAsync(dlist, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
     MHD_CUDA(cudaMemcpyAsync(dparams, hparams.data(), hparams.size() * sizeof(SlotParams), cudaMemcpyHostToDevice, stream));
     list_dirty = false;
@@ -1071,7 +1074,7 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   MHD_CUDA(cudaMalloc(&h->diag_partial, (size_t)s.diag_blocks * kDiagSlots * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->diag_out, 16 * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->dparams, c * sizeof(SlotParams)));
-  MHD_CUDA(cudaMalloc(&h->dlist, (2 * c + 2) * sizeof(int)));
+  MHD_CUDA(cudaMalloc(&h->dlist, (3 * c + 2) * sizeof(int)));
   MHD_CUDA(cudaMalloc(&h->dvmax, 2 * c * sizeof(unsigned int)));
   MHD_CUDA(cudaMalloc(&h->dtime, c * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->dstep, c * sizeof(long long)));

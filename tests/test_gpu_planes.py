@@ -132,3 +132,24 @@ def test_vars_arrays_in_place_and_replaced(pkg, mo, order, dtype):
         assert prob.vars.ux is arrays[0] and prob.vars.by is arrays[1]
         for i, name in enumerate(pkg.FIELDS):
             assert np.array_equal(getattr(prob.vars, name), prob.physical_c(i).T)
+
+
+@pytest.mark.parametrize("n,cap", [(16, 33), (32, 24), (48, 3), (64, 12), (96, 2), (128, 2)])
+def test_single_slot_transforms_of_the_last_slots(pkg, mo, n, cap):
+    """Single-slot launches cover the whole capacity: the instances past the slot stay inside the work
+    lists and the pools, and the last slots' fields and diagnostics equal a single problem's."""
+    g, s, prob, _ = _problem(pkg, mo, n, "mhd")
+    rng = np.random.default_rng(n)
+    f = rng.standard_normal((n, n, n)).astype(np.float32)
+    batch = pkg.Batch(n, cap, stepper="RK4")
+    with prob:
+        for _ in range(cap):
+            batch.add(1e-3, 2e-3, 1e-3)
+        prob.set_physical_c(0, f)
+        for slot in sorted({0, cap // 2, cap - 1}):
+            batch.set_state(slot, s)
+            batch.set_physical(slot, 0, f)
+            assert np.array_equal(batch.get_physical(slot, 0), prob.physical_c(0))
+            a, b = batch.diagnostics(slot), prob.diagnostics()
+            assert (a.E_u, a.E_B, a.H_c, a.nonfinite) == (b.E_u, b.E_B, b.H_c, b.nonfinite)
+    batch.close()
