@@ -6,9 +6,9 @@
 // launches up to n = 64 (x rows, plane_forward, plane_stage) and four at 96 and 128 (plane_inverse
 // and stage_kernel in place of plane_stage), against six with column passes, which at these sizes
 // spend most of their 3 to 5 us on launch, drain and the loads of their first tile.  One RK4 step of
-// one problem, column passes (with stage_kernel) -> plane passes: 32^3 75 -> 43 us, 64^3 101 -> 70,
-// 96^3 172 -> 154, 128^3 335 -> 295; 24 boxes of 32^3 266 -> 170 us per LSRK4 step, 20 of 48^3
-// 536 -> 400, 12 of 64^3 725 -> 500.  Layouts in HBM / L2:
+// one problem, column passes (with stage_kernel) -> plane passes with the x-row tiles and chained
+// graphs of today: 32^3 75 -> 39 us, 64^3 101 -> 63, 96^3 172 -> 153, 128^3 335 -> 290; 24 boxes of
+// 32^3 266 -> 148 us per LSRK4 step, 20 of 48^3 536 -> 366, 12 of 64^3 725 -> 466.  Layouts in HBM / L2:
 //   state    S[f][kx][kz'][ky']   ky' rows padded to k2p (compact fields of stride fs)
 //   planes   R[slot][kx][z][y]    between the plane passes and the x rows (in rowbuf)
 //   products P[slot][kx][kz'][ky'] (in colbuf), as the state
