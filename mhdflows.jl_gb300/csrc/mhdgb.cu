@@ -833,6 +833,16 @@ struct mhd_problem {
   // chained steps need nothing but the next step between two steps: no divergence corrections of the
   // state, no recorded diagnostics
   bool chainable() const { return g.planar && plane_fused(g.n) && !divcorr && diag_freq == 0 && !profiling; }
+  // whether the next nsteps steps run on the chained graph
+  bool chains(int nsteps) const { return chainable() && nsteps >= kChain && graph_steps + nsteps >= kChainAfter; }
+  // The graphs that the next nsteps steps start on.  The timing calls build them before their first event:
+  // an idle device would wait for the capture inside the timed region (16^3, 64 steps: 1.92 ms for 1.75).
+  int build_graphs(int nsteps) {
+    int rc;
+    if (profiling) return MHD_OK;
+    if ((rc = build_graph())) return rc;
+    return chains(nsteps) ? build_chain() : MHD_OK;
+  }
   void advance_clocks() {
     for (int s : active) {
       if (!cfl) t[s] += hparams[s].dt;  // with the on-device CFL the clock lives on the device
@@ -867,11 +877,11 @@ struct mhd_problem {
     int rc;
     if ((rc = sync_lists())) return rc;
     if (active.empty()) return MHD_OK;
-    if (!profiling && (rc = build_graph())) return rc;
-    graph_steps += nsteps;
+    if ((rc = build_graphs(nsteps))) return rc;
     int i = 0;
-    if (chainable() && nsteps >= kChain && graph_steps >= kChainAfter) {
-      if ((rc = build_chain())) return rc;
+    const bool chain = chains(nsteps);
+    graph_steps += nsteps;
+    if (chain) {
       for (; i + kChain <= nsteps; i += kChain) {
         MHD_CUDA(cudaGraphLaunch(graph_chain, stream));
         for (int k = 0; k < kChain; ++k) advance_clocks();
@@ -2093,7 +2103,7 @@ int mhd_time_steps(mhd_handle h, int nsteps, double* ms) {
   if (rc) return rc;
   if (!ms) return fail(MHD_ERR_INVALID, "null output");
   if ((rc = h->sync_lists())) return rc;
-  if (!h->profiling && (rc = h->build_graph())) return rc;
+  if ((rc = h->build_graphs(nsteps))) return rc;
   cudaEvent_t a, b;
   MHD_CUDA(cudaEventCreate(&a));
   MHD_CUDA(cudaEventCreate(&b));
