@@ -2051,22 +2051,39 @@ int mhd_kernel_class_bytes(mhd_handle h, int cls, double* bytes) {
   const double inst = (double)(h->active.empty() ? 1 : h->active.size());
   const double state_field = k2 * k2 * kx * c;
   double b = 0;
-  // state arrays (6 fields each) one epilogue launch touches, averaged over the scheme's stages
-  const double arrays = h->p.scheme == MHD_RK4 ? (3 + 5 + 5 + 4) / 4.0 : (3 + 4 * 4) / 5.0;
+  // state arrays (of all fields) that the stage updates of a launch class touch, averaged over its
+  // launches: the first stage reads the stage state and writes two arrays, the last reads three and writes one
+  const bool rk4 = h->p.scheme == MHD_RK4;
+  const double a_first = 3, a_mid = rk4 ? 5 : 4, a_last = 4;
+  const int stages = rk4 ? 4 : 5;
+  const double a_inv = (a_first + (stages - 2) * a_mid) / (stages - 1);  // every stage but the last
+  const double a_all = (a_first + (stages - 2) * a_mid + a_last) / stages;
   // out-going planes (8 products, 14 with the VP penalty fields) and the VP mask / wall reads
   // the hydrodynamic form moves 3 fields in and 5 products out (6 product slots leave x_fused;
   // with VP 8 slots, the penalty fields in 5..7)
   const bool hd = h->hd_form();
   const bool vp = h->p.vp != 0;
-  const double ns = hd ? (vp ? 8 : 5) : h->ns, nin = hd ? 3 : 6, xout = hd ? (vp ? 8 : 6) : ns;
+  const double ns = hd ? (vp ? 8 : 5) : h->ns, nin = hd ? 3 : 6;
+  const bool tiles = h->ops->xv[h->ops->sel[KC_XFUSED]].tile_fn != nullptr;  // store the five products alone
+  const double xout = hd ? (vp ? 8 : tiles ? 5 : 6) : ns;
   const double vpin = vp ? (h->ops->vp == 2 ? (hd ? 4.0 : 7.0) : 1.0) * n * n * n * 4.0 : 0.0;
+  const double z_field = n * k2 * kx * c, row_field = n * n * kx * c;
+  // plane order: no z-y intermediate, y classes without launches; the z_inverse class is the inverse
+  // plane pass, or the stage updates fused with it (whose last one is the rk_epilogue class)
+  const bool planar = h->g.planar != 0, fused = planar && plane_fused(h->g.n);
+  const double update = ns * state_field, herm = k2 * k2 * c;
   switch (cls) {
-    case KC_ZINV: b = nin * (state_field + n * k2 * kx * c); break;
-    case KC_YINV: b = nin * (n * k2 * kx * c + n * n * kx * c); break;
-    case KC_XFUSED: b = (nin + xout) * n * n * kx * c + vpin; break;
-    case KC_YFWD: b = ns * (n * n * kx * c + n * k2 * kx * c); break;
-    case KC_ZFWD: b = ns * (n * k2 * kx * c + state_field) + 2 * 6 * k2 * k2 * c; break;  // + the kx = 0 Hermitian part
-    case KC_RKEPI: b = ns * state_field + arrays * nin * state_field + nin * k2 * k2 * c; break;
+    case KC_ZINV:
+      b = fused ? update + a_inv * nin * state_field + nin * row_field
+                : nin * (state_field + (planar ? row_field : z_field));
+      break;
+    case KC_YINV: b = planar ? 0 : nin * (z_field + row_field); break;
+    case KC_XFUSED: b = (nin + xout) * row_field + vpin; break;
+    case KC_YFWD: b = planar ? 0 : ns * (row_field + z_field); break;
+    case KC_ZFWD:  // + the kx = 0 Hermitian part (fused: read in the stage update's own plane)
+      b = ns * ((planar ? row_field : z_field) + state_field) + (fused ? 0 : 2 * (planar ? nin : 6) * herm);
+      break;
+    case KC_RKEPI: b = update + (fused ? a_last : a_all) * nin * state_field + (fused ? 0 : nin * herm); break;
     default: b = 0;
   }
   *bytes = b * inst;
