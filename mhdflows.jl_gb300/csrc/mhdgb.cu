@@ -2268,6 +2268,7 @@ int mhd_ensemble_step(mhd_ensemble e, int nsteps) {
     MHD_CUDA(cudaStreamBeginCapture(h0->stream, cudaStreamCaptureModeThreadLocal));
     cudaEventRecord(e->evs[m], h0->stream);
     const std::vector<std::vector<size_t>> lanes = ensemble_lanes(e->hs);
+    std::vector<cudaEvent_t> ends;
     for (const auto& lane : lanes) {
       cudaEvent_t before = e->evs[m];
       for (size_t i : lane) {
@@ -2278,8 +2279,10 @@ int mhd_ensemble_step(mhd_ensemble e, int nsteps) {
         cudaEventRecord(e->evs[i], h->stream);
         before = e->evs[i];
       }
-      if (before != e->evs[m]) cudaStreamWaitEvent(h0->stream, before, 0);
+      if (before != e->evs[m]) ends.push_back(before);
     }
+    // joins come last: member 0 steps on the stream that they hold up
+    for (cudaEvent_t ev : ends) cudaStreamWaitEvent(h0->stream, ev, 0);
     cudaError_t err = cudaStreamEndCapture(h0->stream, &gr);
     if (rc) { if (gr) cudaGraphDestroy(gr); return rc; }
     if (err != cudaSuccess) return fail(MHD_ERR_CUDA, std::string("ensemble capture: ") + cudaGetErrorString(err));
