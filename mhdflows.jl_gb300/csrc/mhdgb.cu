@@ -2179,11 +2179,13 @@ int mhd_select_variant(mhd_handle h, int cls, int idx) {
 struct mhd_ensemble_s {
   std::vector<mhd_handle> hs;
   std::vector<int> versions;
+  std::vector<std::vector<size_t>> lanes;  // of the captured graph
   cudaGraphExec_t graph = nullptr;
   std::vector<cudaEvent_t> evs;
   ~mhd_ensemble_s() {
     if (graph) cudaGraphExecDestroy(graph);
-    for (auto e : evs) cudaEventDestroy(e);
+    for (auto e : evs)
+      if (e) cudaEventDestroy(e);
   }
 };
 
@@ -2254,22 +2256,26 @@ int mhd_ensemble_step(mhd_ensemble e, int nsteps) {
   {
     std::vector<int> v;
     for (auto h : e->hs) v.push_back(h->graph_version);
-    if (e->graph && v != e->versions) {  // a member changed what one of its steps launches
+    std::vector<std::vector<size_t>> lanes = ensemble_lanes(e->hs);
+    // a member changed what one of its steps launches, or its boxes were added or removed so that it
+    // belongs to another lane
+    if (e->graph && (v != e->versions || lanes != e->lanes)) {
       cudaGraphExecDestroy(e->graph);
       e->graph = nullptr;
     }
     e->versions = v;
+    e->lanes = lanes;
   }
   if (!e->graph) {
     const size_t m = e->hs.size();
-    e->evs.resize(m + 1);
-    for (auto& ev : e->evs) MHD_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    e->evs.resize(m + 1, nullptr);
+    for (auto& ev : e->evs)
+      if (!ev) MHD_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     cudaGraph_t gr = nullptr;
     MHD_CUDA(cudaStreamBeginCapture(h0->stream, cudaStreamCaptureModeThreadLocal));
     cudaEventRecord(e->evs[m], h0->stream);
-    const std::vector<std::vector<size_t>> lanes = ensemble_lanes(e->hs);
     std::vector<cudaEvent_t> ends;
-    for (const auto& lane : lanes) {
+    for (const auto& lane : e->lanes) {
       cudaEvent_t before = e->evs[m];
       for (size_t i : lane) {
         if (rc != MHD_OK) break;
