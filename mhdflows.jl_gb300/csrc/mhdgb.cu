@@ -2191,12 +2191,15 @@ struct mhd_ensemble_s {
 
 // Members that step one after another; the lanes step at the same time.  A member of kLaneFull points or more
 // fills the GPU with every launch: more than two of those at once only take L2 and SMs from each other, so
-// they alternate, by size, over two lanes.  A smaller one leaves SMs idle and keeps a lane of its own.  Smaller members
-// come first: their blocks would wait behind a larger one's (5 % at the first mix below, 12 at the last but one).  Ten
-// LSRK4 steps, all members at once against two lanes: 24 x 32^3, 20 x 48^3, 12 x 64^3, 8 x 96^3 (0.8 to
-// 7.1 M points) 23.0 and 21.7 ms; 24, 20, 12, 2 boxes 14.2 and 12.2; 12, 10, 6, 4 boxes 12.1 and 11.0; but
-// 2, 2, 2, 1 boxes (0.07 to 0.9 M) 3.05 and 3.6, and 24 x 32^3, 1 x 64^3, 3 x 96^3 6.1 and 6.6.
-constexpr long long kLaneFull = 500000;
+// they alternate, by size, over two lanes.  A smaller one leaves SMs idle and keeps a lane of its own.  Where
+// the line lies, us a LSRK4 step on two lanes and with every member in its own (members in M points):
+//   0.52, 0.66, 0.66       343 and 266      0.79, 0.88, 0.88, 1.05  569 and 610
+//   0.66, 0.79, 0.88       432 and 374      0.88, 1.05, 1.05, 1.11  645 and 694
+//   0.79, 1.77, 2.2, 3.1  1205 and 1406     2.1, 2.2, 2.6, 2.7     1488 and 1714
+//   0.79, 2.2, 3.1, 7.1   2168 and 2346     1.05, 1.77, 2.1         791 and 776
+// 24 x 32^3 (0.79) beside the other three of a mix took 1273 for 1205 in the third row, 2155 for 2168 in the
+// fourth.  The order in which the lanes are issued changes nothing (2342 and 2350).
+constexpr long long kLaneFull = 700000;
 static std::vector<std::vector<size_t>> ensemble_lanes(const std::vector<mhd_handle>& hs) {
   auto points = [&](size_t i) { return (long long)hs[i]->active.size() * hs[i]->g.n * hs[i]->g.n * hs[i]->g.n; };
   std::vector<size_t> order(hs.size());
