@@ -219,7 +219,7 @@ std::string tune_file() {
   return "";
 }
 
-std::string tune_key(int device, int n, int prec, int vp, int hd = 0) {
+std::string tune_key(int device, int n, int prec, int vp, int hd) {
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return "";
   std::string name(prop.name);
@@ -763,6 +763,7 @@ struct mhd_problem {
     for (int c = 0; c < kTunedClasses; ++c) v.push_back(ops->variant_name(c, ops->sel[c]));
     return v;
   }
+  std::string tuned_key() const { return tune_key(device, g.n, p.precision, ops->vp, ops->hd); }
   int apply_names(const std::vector<std::string>& names) {
     if ((int)names.size() != kTunedClasses) return MHD_ERR_INVALID;
     int saved[kTunedClasses];
@@ -780,7 +781,7 @@ struct mhd_problem {
     if (profiling) return fail(MHD_ERR_STATE, "autotune does not run with per-kernel profiling enabled");
     int rc;
     if ((rc = sync_lists())) return rc;
-    const std::string key = tune_key(device, g.n, p.precision, ops->vp, ops->hd);
+    const std::string key = tuned_key();
     std::vector<std::string> names;
     if (!force && !key.empty() && tuned_lookup(key, &names) && apply_names(names) == MHD_OK) return MHD_OK;
     if (active.empty()) return fail(MHD_ERR_STATE, "autotune needs at least one active slot");
@@ -1065,7 +1066,7 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   {
     // a selection the autotuner made earlier for this device and grid size (this process or the
     // tuning file); the defaults otherwise
-    const std::string key = tune_key(h->device, h->g.n, params->precision, h->ops->vp, h->ops->hd);
+    const std::string key = h->tuned_key();
     std::vector<std::string> names;
     if (!key.empty() && tuned_lookup(key, &names)) h->apply_names(names);
   }
@@ -1746,7 +1747,7 @@ int mhd_slot_set_vp(mhd_handle h, int slot, const float* chi, const float* U0, c
   if (mode != h->ops->vp) {
     if ((rc = h->ops->set_vp(mode))) return rc;
     // a tuned selection of the new form, if one is known
-    const std::string key = tune_key(h->device, h->g.n, h->p.precision, mode);
+    const std::string key = h->tuned_key();
     std::vector<std::string> names;
     if (!key.empty() && tuned_lookup(key, &names)) h->apply_names(names);
     h->invalidate_graph();
