@@ -313,9 +313,11 @@ int mhd_set_div_correction(mhd_handle h, int on);
  * scratch buffers (the state is not touched; at least one slot must be active) and selects the
  * fastest of each class.  The result is kept for the process and appended to a tuning file
  * ($MHDGB_TUNE_CACHE, else $XDG_CACHE_HOME/mhdgb/tune.txt, else $HOME/.cache/mhdgb/tune.txt;
- * MHDGB_TUNE_CACHE="" disables the file), keyed by device name, SM count and n; handles created
- * later for the same key start from it.  Without MHD_TUNE_FORCE a known result is applied
- * without timing.  Every variant computes the same transforms; results agree to FP32 rounding. */
+ * MHDGB_TUNE_CACHE="" disables the file), keyed by device name, SM count, n, precision, penalisation
+ * and field set, and up to n = 128 apart for single problems and batches, which share the x rows (their
+ * variants round differently); handles created later for the same key start from it.  Without
+ * MHD_TUNE_FORCE a known result is applied without timing.  Every variant computes the same
+ * transforms; results agree to FP32 rounding. */
 #define MHD_TUNE_FORCE 1     /* time the candidates even if a result is known */
 #define MHD_TUNE_NO_FILE 2   /* do not append to the tuning file */
 int mhd_autotune(mhd_handle h, int flags);

@@ -201,10 +201,15 @@ namespace {
 
 // ------------------------------------------------------------------------------------------
 // Autotuner results: the selected variant name of each tuned kernel class, keyed by device
-// (name and SM count) and grid size.  Kept for the process and, unless disabled, in a text file
+// (name and SM count), grid size, precision, penalisation and field set.  In plane order batches
+// (OpsBase::batch) have entries of their own, marked "b": the fastest plane variants are opposite ones (64^3
+// inverse 9.9 us with 512 threads and 13.6 with 192 for one problem, 54 and 42 for twelve) and give the
+// same bits.  The x rows round differently from variant to variant, so the two entries share that class and
+// a slot's results stay a single problem's; so do column variants, and there is one entry for both.
+// Kept for the process and, unless disabled, in a text file
 // ($MHDGB_TUNE_CACHE, else $XDG_CACHE_HOME/mhdgb/tune.txt, else $HOME/.cache/mhdgb/tune.txt; an
-// empty $MHDGB_TUNE_CACHE turns the file off).  One line per entry:
-//   <device name>|<sm count>|<n>|<variant of z_inverse>|...|<variant of z_forward>
+// empty $MHDGB_TUNE_CACHE turns the file off).  One line per entry, <key> = n with its marks:
+//   <device name>|<sm count>|<key>|<variant of z_inverse>|...|<variant of z_forward>
 // ------------------------------------------------------------------------------------------
 std::mutex g_tune_mtx;
 std::map<std::string, std::vector<std::string>> g_tuned;
@@ -763,7 +768,27 @@ struct mhd_problem {
     for (int c = 0; c < kTunedClasses; ++c) v.push_back(ops->variant_name(c, ops->sel[c]));
     return v;
   }
-  std::string tuned_key() const { return tune_key(device, g.n, p.precision, ops->vp, ops->hd); }
+  // keys of this handle's entry of the tuned selections and of the one it shares the x rows with ("": none)
+  struct TuneKeys { std::string own, other; };
+  TuneKeys tune_keys() const {
+    const std::string key = tune_key(device, g.n, p.precision, ops->vp, ops->hd);
+    if (key.empty() || !g.planar) return {key, ""};
+    return ops->batch ? TuneKeys{key + "b", key} : TuneKeys{key, key + "b"};
+  }
+  static bool known(const std::string& key, std::vector<std::string>* names) {
+    return !key.empty() && tuned_lookup(key, names) && (int)names->size() == kTunedClasses;
+  }
+  // the selection known for this handle, if there is one; else the x rows of the other entry alone
+  bool apply_known(const TuneKeys& k) {
+    std::vector<std::string> names, other;
+    if (known(k.own, &names) && apply_names(names) == MHD_OK) return true;
+    if (known(k.other, &other)) {
+      names = selected_names();
+      names[KC_XFUSED] = other[KC_XFUSED];
+      apply_names(names);
+    }
+    return false;
+  }
   int apply_names(const std::vector<std::string>& names) {
     if ((int)names.size() != kTunedClasses) return MHD_ERR_INVALID;
     int saved[kTunedClasses];
@@ -781,19 +806,27 @@ struct mhd_problem {
     if (profiling) return fail(MHD_ERR_STATE, "autotune does not run with per-kernel profiling enabled");
     int rc;
     if ((rc = sync_lists())) return rc;
-    const std::string key = tuned_key();
-    std::vector<std::string> names;
-    if (!force && !key.empty() && tuned_lookup(key, &names) && apply_names(names) == MHD_OK) return MHD_OK;
+    const TuneKeys keys = tune_keys();
+    if (!force && apply_known(keys)) return MHD_OK;
     if (active.empty()) return fail(MHD_ERR_STATE, "autotune needs at least one active slot");
     std::vector<std::vector<double>> best;
     if ((rc = tune_rounds(best))) return rc;
+    std::vector<std::string> other;
+    const bool shared = known(keys.other, &other);
+    const bool keep_x = !force && shared && other[KC_XFUSED] == selected_names()[KC_XFUSED];
     for (int c = 0; c < kTunedClasses; ++c) {
+      if (c == KC_XFUSED && keep_x) continue;
       int pick = ops->sel[c];
       for (int i = 0; i < (int)best[c].size(); ++i)
         if (best[c][i] < best[c][pick]) pick = i;
       ops->sel[c] = pick;
     }
-    if (!key.empty()) tuned_store(key, selected_names(), persist);
+    const std::vector<std::string> names = selected_names();
+    if (!keys.own.empty()) tuned_store(keys.own, names, persist);
+    if (shared && other[KC_XFUSED] != names[KC_XFUSED]) {
+      other[KC_XFUSED] = names[KC_XFUSED];
+      tuned_store(keys.other, other, persist);
+    }
     invalidate_graph();
     return MHD_OK;
   }
@@ -1066,9 +1099,7 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   {
     // a selection the autotuner made earlier for this device and grid size (this process or the
     // tuning file); the defaults otherwise
-    const std::string key = h->tuned_key();
-    std::vector<std::string> names;
-    if (!key.empty() && tuned_lookup(key, &names)) h->apply_names(names);
+    h->apply_known(h->tune_keys());
   }
   MHD_CUDA(cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking));
   h->stream = h->own_stream;
@@ -1747,9 +1778,7 @@ int mhd_slot_set_vp(mhd_handle h, int slot, const float* chi, const float* U0, c
   if (mode != h->ops->vp) {
     if ((rc = h->ops->set_vp(mode))) return rc;
     // a tuned selection of the new form, if one is known
-    const std::string key = h->tuned_key();
-    std::vector<std::string> names;
-    if (!key.empty() && tuned_lookup(key, &names)) h->apply_names(names);
+    h->apply_known(h->tune_keys());
     h->invalidate_graph();
   }
   MHD_CUDA(cudaStreamSynchronize(h->stream));
