@@ -1093,7 +1093,7 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   h->ops->hd = h->hd_form() ? 1 : 0;
   h->ops->planar = !h->ops->pv.empty() && params->precision == MHD_PREC_FP32;
   h->g.planar = h->ops->planar ? 1 : 0;
-  h->ops->batch = cap > 1;
+  h->ops->batch = cap >= kBatchCapacity;
   if ((rc = h->ops->setup(h->g))) return rc;
   if (params->vp && (rc = h->ops->set_vp(1))) return rc;  // mask only until walls are set
   {

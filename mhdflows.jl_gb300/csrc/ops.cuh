@@ -103,6 +103,12 @@ struct PlaneVariant {
   int pref = 0;  // default of: bit 0 inverse, bit 1 forward of a single problem; bits 2, 3 of a batch
 };
 
+// Capacity from which a handle takes the plane variants of batches.  One LSRK4 step with the variants of single
+// problems and with those of batches, us: 48^3 2 boxes 80 and 83, 3 boxes 89 and 91, 4 boxes 119 and 105, 6 boxes
+// 147 and 129; 64^3 2 boxes 117 and 125, 3 boxes 155 and 149, 4 boxes 191 and 173.  What the classes hold is
+// not known when they are made: one box in a class of 24 takes 74 and 78 at 48^3, 116 and 110 at 64^3.
+constexpr int kBatchCapacity = 3;
+
 class OpsBase {
  public:
   virtual ~OpsBase();
@@ -141,7 +147,7 @@ class OpsBase {
   // plane order (set before setup): the column classes are the plane passes, y_inverse and
   // y_forward being part of z_inverse's and z_forward's launches
   bool planar = false;
-  bool batch = false;  // capacity above 1 (set before setup): picks the default plane variants
+  bool batch = false;  // kBatchCapacity or more (set before setup): picks the default plane variants
   mutable std::vector<PlaneVariant> pv;
   int sel[kTunedClasses] = {0, 0, 0, 0, 0};  // selected variant of each tuned class
   int variant_count(int cls) const;

@@ -136,3 +136,13 @@ with single(nx=n) as p:
 with pkg.Batch(n, 8) as b:
     assert names(b) == dict(many, x_fused=new["x_fused"])
 """)
+
+
+@pytest.mark.parametrize("n", [48, 64])
+def test_line_between_single_and_batch_defaults(tmp_path, n):
+    """Batches of two take the single problem's plane variants, batches of three the batch's."""
+    _run(tmp_path, f"n = {n}" + """
+with single(nx=n) as p, pkg.Batch(n, 1) as a, pkg.Batch(n, 2) as b, pkg.Batch(n, 3) as c, pkg.Batch(n, 24) as d:
+    assert names(p) == names(a) == names(b)
+    assert names(c) == names(d) != names(p)
+""")
