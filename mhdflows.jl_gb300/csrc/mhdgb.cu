@@ -447,20 +447,21 @@ struct mhd_problem {
     own_stream = nullptr;
   }
 
-  // device work lists: dlist[0..cap) active, dlist[cap..3cap) identity, dlist[3cap] active count, dlist[3cap+1] = 1.
-  // Every kernel may look up any instance below the capacity, active or not (the plane and stage kernels
-  // issue their first loads before they know the count): the entries past the active ones are
-  // slot 0, and slot_ref's list, which starts at the slot's own entry, runs on with the last slot.
-  BatchRef active_ref() const { return BatchRef{dlist, dlist + 3 * cap, cap == 1}; }
-  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 3 * cap + 1, cap == 1}; }
+  // device work lists: dlist[0..cap) active, dlist[cap..2cap) identity, dlist[2cap] active count, dlist[2cap+1] = 1.
+  // A kernel may look up any instance its launch covers, active or not (the plane and stage kernels issue
+  // their first loads before they know the count): the entries past the active ones are slot 0.  A
+  // single slot's launch covers that slot alone.  (Over the capacity, the plane passes of one slot of 4096
+  // of 16^3 took 15.7 us for 5.6, of 512 of 32^3 7.6 for 5.6.)
+  BatchRef active_ref() const { return BatchRef{dlist, dlist + 2 * cap, cap == 1, cap}; }
+  BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 2 * cap + 1, cap == 1, 1}; }
 
   int sync_lists() {
     if (!list_dirty) return MHD_OK;
-    std::vector<int> h(3 * cap + 2, 0);
+    std::vector<int> h(2 * cap + 2, 0);
     for (size_t i = 0; i < active.size(); ++i) h[i] = active[i];
-    for (int i = 0; i < 2 * cap; ++i) h[cap + i] = std::min(i, cap - 1);
-    h[3 * cap] = (int)active.size();
-    h[3 * cap + 1] = 1;
+    for (int i = 0; i < cap; ++i) h[cap + i] = i;
+    h[2 * cap] = (int)active.size();
+    h[2 * cap + 1] = 1;
     MHD_CUDA(cudaMemcpyAsync(dlist, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
     MHD_CUDA(cudaMemcpyAsync(dparams, hparams.data(), hparams.size() * sizeof(SlotParams), cudaMemcpyHostToDevice, stream));
     list_dirty = false;
@@ -513,20 +514,20 @@ struct mhd_problem {
     ColArgs a{src, colbuf, FS(), (long long)g.kxp, (long long)g.k2 * g.kxp, (long long)g.kxp, SLK(), AZ(), sI, sz.colbuf};
     // the maps cover the fields of a pool from its first on
     const TmaPass* tp = sI == ST() ? (src == sol ? &tm_zinv_sol : src == xs ? &tm_zinv_xs : nullptr) : nullptr;
-    return launch(KC_ZINV, [&] { ops->col(KC_ZINV, a, g, g.k2, nf, br, cap, stream, tp, &tm_zfwd); });
+    return launch(KC_ZINV, [&] { ops->col(KC_ZINV, a, g, g.k2, nf, br, stream, tp, &tm_zfwd); });
   }
   int y_inverse(int nf, BatchRef br) {
     ColArgs a{colbuf, rowbuf, (long long)g.kxp, AZ(), SLK(), (long long)g.kxp, BZ(), SLK(), sz.colbuf, sz.rowbuf};
-    return launch(KC_YINV, [&] { ops->col(KC_YINV, a, g, g.n, nf, br, cap, stream, &tm_yinv, &tm_yfwd); });
+    return launch(KC_YINV, [&] { ops->col(KC_YINV, a, g, g.n, nf, br, stream, &tm_yinv, &tm_yfwd); });
   }
   int x_fused(BatchRef br, unsigned int* vmax) {
     // the six field rows of a physical row are contiguous (slot stride == kxp)
     const VpRef vp{vchi, vwall, sz.phys};
-    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, row_stride(), row_slot(), sz.rowbuf, br, cap, vmax, vp, derr, stream, &tm_plane); });
+    return launch(KC_XFUSED, [&] { ops->x_fused(rowbuf, g, row_stride(), row_slot(), sz.rowbuf, br, vmax, vp, derr, stream, &tm_plane); });
   }
   int y_forward(int nf, BatchRef br) {
     ColArgs a{rowbuf, colbuf, (long long)g.kxp, BZ(), SLK(), (long long)g.kxp, AZ(), SLK(), sz.rowbuf, sz.colbuf};
-    return launch(KC_YFWD, [&] { ops->col(KC_YFWD, a, g, g.n, nf, br, cap, stream, &tm_yfwd, &tm_yinv); });
+    return launch(KC_YFWD, [&] { ops->col(KC_YFWD, a, g, g.n, nf, br, stream, &tm_yfwd, &tm_yinv); });
   }
   // colbuf slots -> compact planes (nf fields/products) at dst + slot*dI, pruned output
   // hx: the stage state whose kx = 0 Hermitian part the pass also writes into aux (the
@@ -540,7 +541,7 @@ struct mhd_problem {
     a.hoI = FS();
     // the map of the destination covers the product planes in rowbuf only
     const TmaPass* to = dst == rowbuf && dI == sz.rowbuf ? &tm_prod : nullptr;
-    return launch(KC_ZFWD, [&] { ops->col(KC_ZFWD, a, g, g.k2, nf, br, cap, stream, &tm_zfwd, to); });
+    return launch(KC_ZFWD, [&] { ops->col(KC_ZFWD, a, g, g.k2, nf, br, stream, &tm_zfwd, to); });
   }
   // ---- plane order (small grids): planes R[slot][kx][z][y] in rowbuf, products in colbuf
   // compact fields (src + slot*sI, nf fields at stride FS) -> R planes 0..nf-1
@@ -548,13 +549,13 @@ struct mhd_problem {
     // where the stage update is fused with the inverse pass, that launch is the tuned z_inverse class
     const int cls = plane_fused(g.n) ? KC_OTHER : KC_ZINV;
     const PlaneArgs a{src, rowbuf, sI, sz.rowbuf, FS(), nullptr, nullptr, 0, 0, 0};
-    return launch(cls, [&] { ops->plane_inverse(a, g, nf, br, cap, stream); });
+    return launch(cls, [&] { ops->plane_inverse(a, g, nf, br, stream); });
   }
   // R planes 0..nf-1 -> compact planes at dst + slot*dI
   // hx: as z_forward's
   int plane_forward(float2* dst, long long dI, int nf, BatchRef br, const float2* hx = nullptr) {
     const PlaneArgs a{rowbuf, dst, sz.rowbuf, dI, FS(), hx, aux, ST(), FS(), nfields()};
-    return launch(KC_ZFWD, [&] { ops->plane_forward(a, g, nf, br, cap, stream); });
+    return launch(KC_ZFWD, [&] { ops->plane_forward(a, g, nf, br, stream); });
   }
   // strides of the physical rows in rowbuf
   long long row_stride() const { return g.planar ? 1 : SLK(); }
@@ -598,7 +599,7 @@ struct mhd_problem {
       a.prod = colbuf;
       a.prodI = sz.colbuf;
     }
-    const dim3 grid((unsigned)((field_elems(g) / 2 + kStageThreads - 1) / kStageThreads), hd_form() ? 1 : 2, cap);
+    const dim3 grid((unsigned)((field_elems(g) / 2 + kStageThreads - 1) / kStageThreads), hd_form() ? 1 : 2, br.most);
     return launch(KC_RKEPI, [&] {
       if (hd_form()) launch_epilogue<true, true>(op, grid, a, br);
       else if (a.vpen || a.forced) launch_epilogue<true, false>(op, grid, a, br);
@@ -618,8 +619,8 @@ struct mhd_problem {
     }
   }
   // DivVCorrection! / DivBCorrection! of the slots in br (mask: 1 u, 2 B)
-  int div_correct(BatchRef br, int ninst, int mask) {
-    const dim3 grid((unsigned)((field_elems(g) + 255) / 256), ninst);
+  int div_correct(BatchRef br, int mask) {
+    const dim3 grid((unsigned)((field_elems(g) + 255) / 256), br.most);
     return launch(KC_OTHER, [&] { div_correct_kernel<<<grid, 256, 0, stream>>>(sol, g, FS(), ST(), br, mask); });
   }
   // stage: right-hand-side evaluation within the step (7 outside a step)
@@ -639,7 +640,7 @@ struct mhd_problem {
       a.prod = colbuf;
       a.prodI = sz.colbuf;
       const PlaneArgs pa{nullptr, rowbuf, 0, sz.rowbuf, FS(), nullptr, nullptr, 0, 0, 0};
-      return launch(inv ? KC_ZINV : KC_RKEPI, [&] { ops->plane_stage(a, pa, g, nin, inv, br, cap, stream); });
+      return launch(inv ? KC_ZINV : KC_RKEPI, [&] { ops->plane_stage(a, pa, g, nin, inv, br, stream); });
     }
     if ((rc = z_inverse(X, ST(), nin, br))) return rc;
     if ((rc = y_inverse(nin, br))) return rc;
@@ -668,7 +669,7 @@ struct mhd_problem {
     if (divcorr) {
       // TimeIntegrator! with VP (src/integrator.jl:118-122): DivVCorrection!, and DivBCorrection!
       // for MHD, after every step; they also refresh vars, which the next getCFL! reads
-      if ((rc = div_correct(br, cap, p.hydro_only ? 1 : 3))) return rc;
+      if ((rc = div_correct(br, p.hydro_only ? 1 : 3))) return rc;
       if (cfl && (rc = cfl_prime())) return rc;
     }
     if (cfl && (rc = cfl_update(1))) return rc;
@@ -1116,7 +1117,7 @@ int create_class(const mhd_params* params, int cap, mhd_handle* out) {
   MHD_CUDA(cudaMalloc(&h->diag_partial, (size_t)s.diag_blocks * kDiagSlots * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->diag_out, 16 * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->dparams, c * sizeof(SlotParams)));
-  MHD_CUDA(cudaMalloc(&h->dlist, (3 * c + 2) * sizeof(int)));
+  MHD_CUDA(cudaMalloc(&h->dlist, (2 * c + 2) * sizeof(int)));
   MHD_CUDA(cudaMalloc(&h->dvmax, 2 * c * sizeof(unsigned int)));
   MHD_CUDA(cudaMalloc(&h->dtime, c * sizeof(double)));
   MHD_CUDA(cudaMalloc(&h->dstep, c * sizeof(long long)));
@@ -1794,7 +1795,7 @@ int mhd_slot_div_correct(mhd_handle h, int slot, int fields) {
   if (rc) return rc;
   if (fields < 0 || fields > 3) return fail(MHD_ERR_INVALID, "fields must be a mask of MHD_DIV_U and MHD_DIV_B");
   if (h->p.hydro_only) fields &= MHD_DIV_U;
-  if (fields && (rc = h->div_correct(h->slot_ref(slot), 1, fields))) return rc;
+  if (fields && (rc = h->div_correct(h->slot_ref(slot), fields))) return rc;
   MHD_CUDA(cudaStreamSynchronize(h->stream));
   return MHD_OK;
 }

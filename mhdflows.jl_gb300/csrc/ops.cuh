@@ -113,19 +113,18 @@ class OpsBase {
  public:
   virtual ~OpsBase();
   int setup(const Geom& g);
-  // cap: upper bound of the active instances (the grid covers cap instances; the kernels read
-  // the actual count from the BatchRef)
+  // the grid covers br.most instances; the kernels read the actual count
   // tp, to: the TMA source and destination of this call (nullptr or !ok: a selection that needs it falls back
   // to variant 0)
-  void col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, int cap, cudaStream_t s,
+  void col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, cudaStream_t s,
            const TmaPass* tp = nullptr, const TmaPass* to = nullptr) const;
   void x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride, BatchRef br,
-               int cap, unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp = nullptr) const;
+               unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp = nullptr) const;
   // plane passes: forward transforms of nslots planes per kx mode; stage update (a.op) of nf
-  // fields and, with inv, their inverse transforms.  cap as in col.
-  void plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, int cap, cudaStream_t s) const;
-  void plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, int cap, cudaStream_t s) const;
-  void plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, int nf, bool inv, BatchRef br, int cap,
+  // fields and, with inv, their inverse transforms.
+  void plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, cudaStream_t s) const;
+  void plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, cudaStream_t s) const;
+  void plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, int nf, bool inv, BatchRef br,
                    cudaStream_t s) const;
   // x rows in plane order by TMA tiles, map over the R planes (a variant that reads the planes directly
   // when the map could not be encoded)

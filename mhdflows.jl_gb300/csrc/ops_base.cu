@@ -178,14 +178,14 @@ int OpsBase::select_by_name(int cls, const std::string& name) {
   return report_error(MHD_ERR_INVALID, "no kernel variant named " + name);
 }
 
-void OpsBase::col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, int cap,
+void OpsBase::col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br,
                   cudaStream_t s, const TmaPass* tp, const TmaPass* to) const {
   const ColVariant& sv = cv[sel[cls]];
   const bool in = tp && tp->ok, out = to && to->ok;
   const ColVariant& c = (sv.inv_tma && !in) || (sv.inv_pair && !(in && out)) ? cv[0] : sv;
   const bool inv = is_inv(cls);
   const ColWork w{(g.kx + c.tx - 1) / c.tx, outer, nf, inv ? g.k2 : n};
-  const long long total = (long long)cap * w.tiles_x * w.outer * w.nf;
+  const long long total = (long long)br.most * w.tiles_x * w.outer * w.nf;
   const int ctas = inv ? c.ctas_inv : c.ctas_fwd;
   const int grid = (int)(total < ctas ? total : ctas);
   if (c.inv_pair) {
@@ -200,37 +200,37 @@ void OpsBase::col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, B
   f<<<grid, c.threads, c.smem, s>>>(a, g, w, br, tw_dev + c.tw);
 }
 
-void OpsBase::plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, int cap, cudaStream_t s) const {
+void OpsBase::plane_forward(const PlaneArgs& a, const Geom& g, int nslots, BatchRef br, cudaStream_t s) const {
   const PlaneVariant& v = pv[sel[KC_ZFWD]];
-  v.fwd<<<dim3(g.kx, nslots, cap), v.threads, v.smem, s>>>(a, g, br, tw_dev + v.tw);
+  v.fwd<<<dim3(g.kx, nslots, br.most), v.threads, v.smem, s>>>(a, g, br, tw_dev + v.tw);
 }
 
-void OpsBase::plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, int cap, cudaStream_t s) const {
+void OpsBase::plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, cudaStream_t s) const {
   const PlaneVariant& v = pv[sel[KC_ZINV]];
-  v.inv<<<dim3(g.kx, nf, cap), v.threads, v.smem, s>>>(a, br, tw_dev + v.tw);
+  v.inv<<<dim3(g.kx, nf, br.most), v.threads, v.smem, s>>>(a, br, tw_dev + v.tw);
 }
 
 void OpsBase::plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, int nf, bool inv, BatchRef br,
-                          int cap, cudaStream_t s) const {
+                          cudaStream_t s) const {
   const PlaneVariant& v = pv[sel[KC_ZINV]];
   const PlaneStageFn f = hd ? v.stage_hd : (a.vpen || a.forced) ? v.stage_gen : v.stage;
-  f<<<dim3(g.kx, nf, cap), v.threads, v.smem, s>>>(a, pa, g, br, inv ? 1 : 0, tw_dev + v.tw);
+  f<<<dim3(g.kx, nf, br.most), v.threads, v.smem, s>>>(a, pa, g, br, inv ? 1 : 0, tw_dev + v.tw);
 }
 
 void OpsBase::x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride,
-                      BatchRef br, int cap, unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp) const {
+                      BatchRef br, unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp) const {
   const XVariant* sv = &xv[sel[KC_XFUSED]];
   if (sv->tile_fn && !(tp && tp->ok))  // no tensor map: the first variant of this form without one
     for (size_t i = 0; i < xv.size(); ++i)
       if (variant_ok(KC_XFUSED, (int)i) && !xv[i].tile_fn) { sv = &xv[i]; break; }
   const XVariant& x = *sv;
   if (x.tile_fn) {
-    const long long tiles = (long long)cap * n * n / x.rpg;
+    const long long tiles = (long long)br.most * n * n / x.rpg;
     x.tile_fn<<<(unsigned)(tiles < x.ctas ? tiles : x.ctas), x.threads, x.smem, s>>>(tp->map, tp->err, br, tw_dev + x.tw,
                                                                                     tw_dev + x.twr, vmax, vp);
     return;
   }
-  const long long groups = (long long)cap * n * n / x.rpg;
+  const long long groups = (long long)br.most * n * n / x.rpg;
   const long long need = (groups + x.groups - 1) / x.groups;
   const int grid = (int)(need < x.ctas ? need : x.ctas);
   const float2* t1 = x.table ? reinterpret_cast<const float2*>(x.table) : tw_dev + x.tw;

@@ -98,6 +98,7 @@ struct BatchRef {
   const int* list;   // active slots
   const int* count;  // number of active slots
   int single;        // capacity 1: the slot is 0 and needs no load in front of the first data address
+  int most;          // instances a launch covers: the count is at most this
   __device__ __forceinline__ int slot(int inst) const { return single ? 0 : list[inst]; }
 };
 
