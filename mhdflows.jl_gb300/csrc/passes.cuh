@@ -100,6 +100,10 @@ struct BatchRef {
   int single;        // capacity 1: the slot is 0 and needs no load in front of the first data address
   int most;          // instances a launch covers: the count is at most this
   __device__ __forceinline__ int slot(int inst) const { return single ? 0 : list[inst]; }
+  // An instance of a batch past its active ones, to be left before the first loads: one box in a class of 16
+  // takes 192 us a step at 96^3, with the loads of the 15 others 244; full classes are equal to 0.4 %.
+  // (A single problem's first loads go ahead of the count, which is tested after them.)
+  __device__ __forceinline__ bool past(int inst, int active) const { return !single && inst >= active; }
 };
 
 // Volume-penalisation inputs of the x rows (src/Solver/VPSolver.jl): per slot the mask chi
