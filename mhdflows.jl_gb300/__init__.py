@@ -385,7 +385,7 @@ def _vars_memory(prob, f):
     """Address of the vars array of field f if the library can write it in place (float32 in
     column-major order, as Vars lays it out), else None: an array of another kind was put there."""
     a = getattr(prob.vars, FIELDS[f])
-    ok = (isinstance(a, np.ndarray) and a.dtype == np.float32 and a.shape == (prob.n,) * 3 and a.flags.f_contiguous
+    ok = (type(a) is np.ndarray and a.dtype == np.float32 and a.shape == (prob.n,) * 3 and a.flags.f_contiguous
           and a.flags.writeable and a.flags.aligned and a.dtype.isnative)
     return a.ctypes.data if ok else None
 
