@@ -161,6 +161,7 @@ class OpsBase {
   bool ready(ColVariant& c, bool inv) const;
   bool preferred(int cls, int i) const;
   int sm_count = 0, smem_limit = 0, kxp = 0;
+  mutable int table_rc = 0;  // why a variant's tables could not be made
   // plain row transforms (staging of set_physical / get_physical / diagnostics)
   C2RFn c2r = nullptr, c2r_plane = nullptr;
   R2CFn r2c = nullptr, r2c_plane = nullptr;

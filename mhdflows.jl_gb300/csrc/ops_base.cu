@@ -46,12 +46,18 @@ bool OpsBase::ready(XVariant& x) const {
   x.smem = x.tile_fn ? x.tile_smem : sizeof(float2) * (size_t)x.groups * x.group_words(kxp);
   if ((int)x.smem > smem_limit) return false;
   if (x.build_table) {
-    if (cudaMalloc(&x.table, x.table_words * sizeof(uint32_t)) != cudaSuccess) {
+    if (!x.table && cudaMalloc(&x.table, x.table_words * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
       x.table = nullptr;
+      x.state = 0;  // asked for again, there may be memory
+      table_rc = MHD_ERR_OOM;
       return false;
     }
-    if (x.build_table(x.table)) return false;
+    if (x.build_table(x.table)) {
+      cudaGetLastError();
+      table_rc = MHD_ERR_CUDA;
+      return false;
+    }
   }
   // max_carveout: the whole unified L1 / shared array as shared memory (two CTAs per SM fit only then)
   if (set_smem(fn, x.smem) ||
@@ -116,6 +122,9 @@ int OpsBase::setup(const Geom& g) {
     while (i < variant_count(cls) && !(preferred(cls, i) && variant_ok(cls, i))) ++i;
     if (i == variant_count(cls))
       for (i = 0; i < variant_count(cls) && !variant_ok(cls, i);) ++i;
+    if (i == variant_count(cls) && cls == KC_XFUSED && table_rc)
+      return report_error(table_rc, table_rc == MHD_ERR_OOM ? "tensor-core tables: out of memory"
+                                                            : "building the tensor-core DFT tables failed");
     if (i == variant_count(cls))
       return report_error(cls == KC_XFUSED && prec ? MHD_ERR_INVALID : MHD_ERR_CUDA,
                           cls == KC_XFUSED && prec ? "no x-row kernel of this precision form for this grid size"
