@@ -230,8 +230,9 @@ int mhd_server_cancel(mhd_server s, long long rid);
 /* device bytes reserved by the server's size classes now, and the peak so far */
 int mhd_server_memory(mhd_server s, double* reserved, double* peak);
 
-/* Ensembles of size classes stepped together: one CUDA graph holds one step of every member,
- * each member on its own stream, so boxes of different sizes run concurrently. */
+/* Ensembles of size classes stepped together: one CUDA graph holds one step of every member.  Members
+ * that leave the GPU partly idle run side by side, members that fill it (700000 points) on two lanes
+ * beside them; the lanes follow the boxes that are in the classes at each call. */
 int mhd_ensemble_create(mhd_handle* handles, int count, mhd_ensemble* out);
 int mhd_ensemble_step(mhd_ensemble e, int nsteps);
 int mhd_ensemble_destroy(mhd_ensemble e);

@@ -637,8 +637,8 @@ class Batch:
 
 
 class Ensemble:
-    """Size classes stepped together: one CUDA graph per step forks every member onto its own
-    stream, so boxes of different sizes advance concurrently."""
+    """Size classes stepped together: one CUDA graph per step runs them side by side, those that fill
+    the GPU on two lanes."""
 
     def __init__(self, batches):
         self._lib = _lib.load()

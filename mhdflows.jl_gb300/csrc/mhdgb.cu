@@ -1016,11 +1016,8 @@ struct mhd_problem {
     if (ops->x_device_error()) return fail(MHD_ERR_CUDA, "a tensor-core completion wait of the x rows timed out on the device");
     return MHD_OK;
   }
-  // Hydrodynamics runs the MHD kernels with B = 0: the epilogue sets the induction right-hand
-  // side to zero, so B stays exactly zero, and the momentum right-hand side is HDcalcN!'s (the
-  // x rows pair uz with bx in one transform, so they see FP32 roundoff in place of bx = 0; its
-  // products enter the momentum at ~1e-14 relative).  Only the three velocity fields cross the
-  // boundary.
+  // hydrodynamics: only the three velocity fields cross the boundary; no step reads or writes B, which
+  // keeps the zeros of its allocation
   int nfields() const { return p.hydro_only ? 3 : 6; }
   // the dedicated hydrodynamic passes (three fields in, five products out; with volume
   // penalisation also the three velocity penalty fields, in the spare slots 5..7)
@@ -2204,8 +2201,8 @@ int mhd_select_variant(mhd_handle h, int cls, int idx) {
 
 // ------------------------------------------------------------------------------------------
 // Ensembles: several size classes stepped concurrently.  One step of every class is captured
-// into a single CUDA graph: the classes fork onto their own streams and join on the first one,
-// so small boxes run alongside large ones instead of one class after another.
+// into a single CUDA graph: the lanes of classes (ensemble_lanes) fork onto the classes' streams and join on
+// the first one's after the last lane, so small boxes run alongside large ones.
 // ------------------------------------------------------------------------------------------
 struct mhd_ensemble_s {
   std::vector<mhd_handle> hs;

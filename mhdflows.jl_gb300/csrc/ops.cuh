@@ -118,6 +118,8 @@ class OpsBase {
   // to variant 0)
   void col(int cls, const ColArgs& a, const Geom& g, int outer, int nf, BatchRef br, cudaStream_t s,
            const TmaPass* tp = nullptr, const TmaPass* to = nullptr) const;
+  // tp: in plane order the tensor map over the R planes, for x rows by TMA tiles (where it could not be
+  // encoded, the first variant of the form that reads the planes directly)
   void x_fused(float2* pool, const Geom& g, long long rowstride, long long slot, long long istride, BatchRef br,
                unsigned int* vmax, VpRef vp, int* err, cudaStream_t s, const TmaPass* tp = nullptr) const;
   // plane passes: forward transforms of nslots planes per kx mode; stage update (a.op) of nf
@@ -126,8 +128,6 @@ class OpsBase {
   void plane_inverse(const PlaneArgs& a, const Geom& g, int nf, BatchRef br, cudaStream_t s) const;
   void plane_stage(const RkArgs& a, const PlaneArgs& pa, const Geom& g, int nf, bool inv, BatchRef br,
                    cudaStream_t s) const;
-  // x rows in plane order by TMA tiles, map over the R planes (a variant that reads the planes directly
-  // when the map could not be encoded)
   void x_c2r(const float2* src, float* dst, const Geom& g, long long srow, float scale, cudaStream_t s) const;
   void x_r2c(const float* src, float2* dst, const Geom& g, long long drow, cudaStream_t s) const;
   // a bounded device wait of the selected x-row kernel that ran out (its table's error word);

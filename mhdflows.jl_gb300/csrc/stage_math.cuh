@@ -39,7 +39,7 @@ struct RkArgs {
   const long long* step; // per-slot step counters (random forcing: call = 8 * step + stage)
   int stage;             // right-hand-side evaluation within the step (7: outside a step)
   float vscale;          // 1/n^3: the penalty planes are n^3 times the reference's rfft
-  int vpen, forced;      // plane passes: penalty planes present, forcing on for some slot
+  int vpen, forced;      // penalty planes present, forcing on for some slot (read by the GENERAL forms)
 };
 
 // ------------------------------------------------------------------------------------------

@@ -125,8 +125,11 @@ __global__ void step_tick_kernel(BatchRef br, long long* steps) {
 constexpr int kCopyThreads = 256;
 
 // Retained modes of the reference layout -> compact state, in the reference's order (kx fastest), so
-// that the reads, which may cross the host link, are contiguous; padding elements of S are never
-// read and keep the zeros of their allocation.  blockIdx.y = f k2 + kz'.
+// that the reads, which may cross the host link, are contiguous.  blockIdx.y = f k2 + kz'.  Padding
+// elements of S are not written here and hold anything: in column order an odd Kx leaves the second
+// half of a row's last pair in the padding (256^3: modes 84 and 85 of 85), which stage_kernel updates with
+// the rest, and the column pairs transform the padding columns of a tile.  No kernel mixes a column with
+// another before the x rows, and those read the kept modes alone.
 __global__ void __launch_bounds__(kCopyThreads) gather_state_kernel(const float2* __restrict__ ref, float2* __restrict__ S,
                                                                     Geom geo) {
   const unsigned int kx = geo.kx, total = (unsigned int)geo.k2 * kx;
