@@ -448,16 +448,15 @@ struct mhd_problem {
   }
 
   // device work lists: dlist[0..cap) active, dlist[cap..2cap) identity, dlist[2cap] active count, dlist[2cap+1] = 1.
-  // A kernel may look up any instance its launch covers, active or not (the plane and stage kernels issue
-  // their first loads before they know the count): the entries past the active ones are slot 0.  A
-  // single slot's launch covers that slot alone.  (Over the capacity, the plane passes of one slot of 4096
-  // of 16^3 took 15.7 us for 5.6, of 512 of 32^3 7.6 for 5.6.)
+  // A kernel may look up any instance its launch covers; the entries past the active ones are 0 or -1
+  // (BatchRef::slot).  A single slot's launch covers that slot alone.  (Over the capacity, the plane passes of
+  // one slot of 4096 of 16^3 took 15.7 us for 5.6, of 512 of 32^3 7.6 for 5.6.)
   BatchRef active_ref() const { return BatchRef{dlist, dlist + 2 * cap, cap == 1, cap}; }
   BatchRef slot_ref(int slot) const { return BatchRef{dlist + cap + slot, dlist + 2 * cap + 1, cap == 1, 1}; }
 
   int sync_lists() {
     if (!list_dirty) return MHD_OK;
-    std::vector<int> h(2 * cap + 2, 0);
+    std::vector<int> h(2 * cap + 2, g.planar && plane_fused(g.n) ? 0 : -1);
     for (size_t i = 0; i < active.size(); ++i) h[i] = active[i];
     for (int i = 0; i < cap; ++i) h[cap + i] = i;
     h[2 * cap] = (int)active.size();

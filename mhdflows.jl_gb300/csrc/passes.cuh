@@ -99,11 +99,13 @@ struct BatchRef {
   const int* count;  // number of active slots
   int single;        // capacity 1: the slot is 0 and needs no load in front of the first data address
   int most;          // instances a launch covers: the count is at most this
+  // The slot of an instance.  Of a batch's instances past the active ones it is -1 where a launch is large
+  // enough for their loads to matter (96^3 and more): the plane and stage kernels, whose grids cover them, return
+  // on it.  One box in a class of 8, us a RK4 step: 96^3 189 -> 170, 128^3 382 -> 327; full classes and single
+  // problems 0.6 % either way (eight boxes RK4 and LSRK4 at 96^3 984 -> 986 and 1201 -> 1208, at 128^3 LSRK4 2616 ->
+  // 2608, one 297 -> 298 and 370 -> 367).  Up to 64^3, where it would save 2 % in such a class and cost a single
+  // problem 0.5, it is 0 and their first loads go to slot 0.
   __device__ __forceinline__ int slot(int inst) const { return single ? 0 : list[inst]; }
-  // An instance of a batch past its active ones, to be left before the first loads: one box in a class of 16
-  // takes 192 us a step at 96^3, with the loads of the 15 others 244; full classes are equal to 0.4 %.
-  // (A single problem's first loads go ahead of the count, which is tested after them.)
-  __device__ __forceinline__ bool past(int inst, int active) const { return !single && inst >= active; }
 };
 
 // Volume-penalisation inputs of the x rows (src/Solver/VPSolver.jl): per slot the mask chi

@@ -162,8 +162,8 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_forward_kernel(PlaneArgs 
 #pragma unroll
       for (int n0 = 0; n0 < P::R0; ++n0) u[d * P::R0 + n0] = s[row * N + g + G * d + P::LI * n0];
   };
-  if (br.past(blockIdx.z, active)) return;
-  // one round: the loads of a single problem come before the test of the instance and do not wait for its count
+  if (!plane_fused(C::N) && slot < 0) return;
+  // one round: the loads come before the test of the instance and do not wait for its count
   constexpr bool ONE = C::RB >= N;
   int r0 = (threadIdx.x >> 5) * C::RPW;
   if (ONE && r0 < N) load(r0 + lane / G);
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_inverse_kernel(PlaneArgs 
   const int active = *br.count, slot = br.slot(blockIdx.z);
   const int x = blockIdx.x, f = blockIdx.y;
   const float2* X = a.src + slot * a.sI + f * a.dF + (long long)x * (C::K2 * C::K2P);
-  if (br.past(blockIdx.z, active)) return;
+  if (!plane_fused(C::N) && slot < 0) return;
   for (int m = threadIdx.x; m < C::K2 * C::K2 / 2; m += C::T) {
     const int jz = m / (C::K2 / 2), jy = 2 * (m % (C::K2 / 2));
     *reinterpret_cast<float4*>(W + plane_freq<C>(jz) * C::S + jy) = *reinterpret_cast<const float4*>(X + jz * C::K2P + jy);
@@ -305,7 +305,6 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_stage_kernel(RkArgs a, Pl
   const int x = blockIdx.x, f = blockIdx.y, t = f / 3, op = a.op;
   const long long so = slot * a.stI + f * a.fs + (long long)x * (K2 * K2P);
   const float2* X = a.X + so;
-  if (br.past(blockIdx.z, active)) return;
   float4 xv[NP], xd[NP];
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(C::T, C::MINB) plane_stage_kernel(RkArgs a, Pl
     if (m < PAIRS) xv[i] = *reinterpret_cast<const float4*>(X + jz * K2P + jy);
     xd[i] = xv[i];
   }
-  if ((int)blockIdx.z >= active) return;  // a single problem: after the first loads, which do not wait for the count
+  if ((int)blockIdx.z >= active) return;  // after the first loads, which do not wait for the count
   if (x == 0) {  // X(-k) = 0 when -k lies in the alias band
 #pragma unroll
     for (int i = 0; i < NP; ++i) {

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo
   const int active = *br.count, slot = br.slot(blockIdx.z);
   int x, jy, jz;
   if (i >= field_elems(geo) || !mode_at(geo, i, x, jy, jz)) return;
-  if (br.past(blockIdx.z, active)) return;
+  if (slot < 0) return;
   const int t = blockIdx.y;
   const long long so = slot * a.stI + 3 * t * a.fs + i;
   const float2* X = a.X + so;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kStageThreads) stage_kernel(RkArgs a, Geom geo
       pn[c] = a.vpen ? __ldcs(reinterpret_cast<const float4*>(prod + pp * a.fs)) : zero4;
     }
   }
-  if ((int)blockIdx.z >= active) return;  // a single problem: after the loads, which do not wait for the count
+  if ((int)blockIdx.z >= active) return;  // after the loads, which do not wait for the count
   const SlotParams sp = a.sp[slot];
   const RkSlot rs{rs0.sol, rs0.acc, rs0.xn, a.hf * sp.dt, sp.dt, sp.dt / 6.f, a.ca, a.cb};
   // the kx = 0 plane diffuses its Hermitian part, H[f][kz'][ky'] (written before X is updated)
