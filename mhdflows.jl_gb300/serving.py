@@ -5,7 +5,7 @@ Requests (n, nu, eta, steps, seed, arrival time) arrive over time.  The server k
 admitted solve's state resident in HBM in a size class (a Batch: slots of one grid size), admits
 a request when its size class has a free slot or a new class fits in the memory budget (the
 budget is charged with the measured device bytes of each class), and advances all active solves
-together: one CUDA graph per tick steps every non-empty class, each on its own stream.  Requests
+together: one CUDA graph per tick steps every non-empty class, side by side.  Requests
 that arrive while others run join at the next tick; finished ones free their slot at once.
 Results do not depend on what else is in the batch (no reduction crosses slots).
 
