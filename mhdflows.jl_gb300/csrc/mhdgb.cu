@@ -862,6 +862,7 @@ struct mhd_problem {
     e = cudaGraphInstantiate(&graph_chain, gr, 0);
     cudaGraphDestroy(gr);
     if (e != cudaSuccess) { graph_chain = nullptr; return fail(MHD_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e)); }
+    MHD_CUDA(cudaGraphUpload(graph_chain, stream));  // else part of its first launch, 35 us
     return MHD_OK;
   }
   // chained steps need nothing but the next step between two steps: no divergence corrections of the
